@@ -1,0 +1,359 @@
+// Host side of the closed-form sweeps (bfvm_kernels_closed.cuh): their
+// constants, and the launches bfvm_solver.cu's sweep() makes under
+// BFVM_PATH_AUTO.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+#include <vector>
+
+#include "bfvm.h"
+#include "bfvm_kernels_closed.cuh"
+#include "bfvm_state.h"
+
+namespace bfvm_rt {
+
+namespace {
+
+int axis_points(const bfvm_solver* m, int a) { return a == 0 ? m->nx : (a == 1 ? m->ny : m->nz); }
+
+// Points per thread: 32 where the line is whole 32-point chunks or has at
+// least six of them, else 16.  A 32-point chunk spreads the per-thread work
+// (indices, carries) over twice the points (y at 256^3 x 10 FP64 415 -> 396
+// us, at 256^3 x 4 FP32 132 -> 98), but a line's last, partial chunk runs the
+// body with bounds checks, a quarter of the threads of a 123-point line (z at
+// 161 x 97 x 123 x 3: 20.2 us at 16 points, 22.9 at 32).
+int closed_chunk(const bfvm_solver* m, int a) {
+  const int n = axis_points(m, a);
+  return n % 32 == 0 || n > 160 ? 32 : 16;
+}
+
+// floor(2^64 / d) + 1 for quot(), 0 for d = 1.
+uint64_t quot_of(uint64_t d) { return d <= 1 ? 0 : ~(uint64_t)0 / d + 1; }
+
+}  // namespace
+
+// Whether the closed-form kernels sweep this axis: the default choice
+// (BFVM_PATH_AUTO, no configuration set on the axis), lines the chunked
+// kernels take, whole lines (a z slab's carries come from the other slabs).
+bool closed_axis(const bfvm_solver* m, int ax) {
+  if (m->path != BFVM_PATH_AUTO || m->axis[ax].user) return false;
+  if (ax == 2 && m->zs_ranks > 0) return false;
+  if (ax == 0 && m->fuse_sources) return false;
+  const int n = axis_points(m, ax);
+  return n <= 1024 && m->NS() / n < ((int64_t)1 << 31);
+}
+
+int closed_axis_chunk(const bfvm_solver* m, int ax) { return closed_chunk(m, ax); }
+
+// Constants of every axis from the coefficients of the Thomas setup
+// (BioFVM_solvers.cpp:105-126: c1 = dt D / dx^2, c2 = dt decay / 3, or / 2
+// for LOD_2D), in extended precision and rounded once.
+void closed_setup(bfvm_solver* m) {
+  const int S = m->S;
+  const double dt = m->setup_dt;
+  for (int a = 0; a < 3; ++a) {
+    const int n = axis_points(m, a);
+    if (n > 1024) continue;
+    const int ch = closed_chunk(m, a), nc = (n + ch - 1) / ch;
+    const bool fp32 = m->math_elem() == 4;
+    const size_t ncst = (size_t)S * 8, count = ncst + (size_t)nc * S * 2;
+    std::vector<double> t(count, 0.0);
+    std::vector<float> tf(fp32 ? 2 * count : 0, 0.0f);
+    for (int s = 0; s < S; ++s) {
+      const long double c1 = (long double)m->h_c1[a][s];
+      const long double c2 = (long double)m->setup_decay[s] * dt / (m->setup_dims == 2 ? 2 : 3);
+      // r = c1 / d with d the larger root of d^2 - (1 + 2 c1 + c2) d + c1^2
+      const long double b = 1 + 2 * c1 + c2;
+      const long double d = (b + std::sqrt((1 + c2) * (1 + c2 + 4 * c1))) / 2;
+      const long double r = fp32 ? (long double)(float)(c1 / d) : (long double)(double)(c1 / d);
+      auto put = [&](size_t i, long double x) {
+        t[i] = (double)x;
+        if (fp32) {
+          tf[2 * i] = (float)x;
+          tf[2 * i + 1] = (float)(x - tf[2 * i]);
+        }
+      };
+      auto power = [&](int k) { return std::pow(r, (long double)k); };
+      const int last = n - (nc - 1) * ch;
+      const long double k[7] = {r, (1 - r) * (1 - r) / (1 + c2), 1 / ((1 - r) * (1 + r)),
+                                power(ch), power(last), power(n), 1 / (1 - power(2 * n))};
+      for (int i = 0; i < 7; ++i) put((size_t)s * 8 + i, k[i]);
+      for (int c = 0; c < nc; ++c) {
+        const size_t i = ncst + ((size_t)c * S + s) * 2;
+        put(i, power(c * ch));
+        put(i + 1, power(n - std::min(n, (c + 1) * ch)));
+      }
+    }
+    if (fp32)
+      upload(m->closed_tab[a], tf, m->stream);
+    else
+      upload(m->closed_tab[a], t, m->stream);
+  }
+}
+
+namespace {
+
+template <typename CT>
+bfvm::ClosedCoef<CT> closed_view(const bfvm_solver* m, int a) {
+  const CT* t = m->closed_tab[a].as<CT>();
+  return {t, t + (size_t)m->S * 8 * (sizeof(CT) == 4 ? 2 : 1)};
+}
+
+// Calls f with each of the flags as a compile-time constant.
+template <typename F, typename... B>
+void with_flags(F&& f, bool b, B... rest) {
+  auto one = [&](auto c) {
+    if constexpr (sizeof...(rest) == 0)
+      f(c);
+    else
+      with_flags([&](auto... cs) { f(c, cs...); }, rest...);
+  };
+  if (b)
+    one(std::true_type());
+  else
+    one(std::false_type());
+}
+
+template <typename T, typename CT, int CH, int MAXT>
+void lines(bfvm_solver* m, const bfvm::ClosedArgs<T, CT>& a, bool ca, dim3 grid, dim3 block,
+           size_t smem) {
+  with_flags(
+      [&](auto dir, auto l1, auto exact) {
+        bfvm::closed_lines_kernel<T, CT, CH, MAXT, decltype(dir)::value, decltype(l1)::value,
+                                  decltype(exact)::value><<<grid, block, smem, m->stream>>>(a);
+      },
+      a.fuse != 0, ca, a.n % CH == 0);
+  check_launch(m);
+}
+
+template <typename T, typename CT>
+void sweep_lines(bfvm_solver* m, int ax, int fuse, int64_t z0, int64_t z1) {
+  const int64_t nx = m->nx, ny = m->ny, nz = m->nz, S = m->S;
+  const int64_t nzp = m->lod_dims == 2 ? 1 : nz;  // planes swept
+  bfvm::ClosedArgs<T, CT> a{};
+  a.p = m->p.as<T>();
+  a.out = m->sweep_out ? static_cast<T*>(m->sweep_out) : a.p;
+  int64_t per_plane = 0;
+  if (ax == 0) {
+    a.n = (int)nx, a.C = (uint32_t)S, a.os = nx * S, a.ls = S, per_plane = ny * S;
+  } else if (ax == 1) {
+    a.n = (int)ny, a.C = (uint32_t)(nx * S), a.os = nx * ny * S, a.ls = nx * S;
+    per_plane = nx * S;
+  } else {
+    a.n = (int)nz, a.C = (uint32_t)(nx * ny * S), a.os = 0, a.ls = nx * ny * S;
+  }
+  a.ncols = (uint32_t)(ax == 2 ? nx * ny * S : per_plane * nzp);
+  if (z1 >= 0 && ax < 2) {  // columns of planes z0 .. z1-1
+    a.col0 = (uint32_t)(z0 * per_plane);
+    a.ncols = (uint32_t)(z1 * per_plane);
+  }
+  a.mC = quot_of(a.C);
+  a.mS = quot_of(S);
+  a.S = (int)S;
+  const int ch = closed_chunk(m, ax), nc = (a.n + ch - 1) / ch;
+  a.cc = closed_view<CT>(m, ax);
+  const DevSegList& dseg = ax == 0 ? m->seg_dir_x : m->seg_dir_y;
+  if (ax == 2 || !dseg.present) fuse = 0;
+  a.fuse = fuse & (bfvm::kFuseDirPro | bfvm::kFuseDirEpi);
+  a.dir = dseg.view();
+  const int W = nc <= 16 ? 32 : 16;
+  const dim3 block(W, nc), grid((unsigned)blocks_for(a.ncols - a.col0, W));
+  const size_t smem = (size_t)2 * nc * W * sizeof(CT);
+  const bool ca = ax == 0 && S * (int)sizeof(T) < 256;
+  if (ch == 16)
+    lines<T, CT, 16, 512>(m, a, ca, grid, block, smem);
+  else if (W * nc <= 256)
+    lines<T, CT, 32, 256>(m, a, ca, grid, block, smem);
+  else
+    lines<T, CT, 32, 512>(m, a, ca, grid, block, smem);
+}
+
+constexpr size_t kTileSmem = 224 * 1024;  // of the 227 KB a block may use
+
+struct TilePlan {
+  bool ok = false;
+  int ch = 0, nc = 0, w = 0, maxt = 0, stages = 0;
+  int box_n = 0, nboxes = 0;     // lines
+  int R = 0, pitch = 0;          // rows
+  int stage_elems = 0;
+  size_t smem = 0;
+  uint32_t tile0 = 0, ntiles = 0;
+};
+
+// The ring of an axis's tiles: 32 columns by n points each, 16 from 257 points
+// on, which keeps two blocks of 256 threads per SM up to 512 points.
+template <typename T, typename CT>
+TilePlan plan_tiles(const bfvm_solver* m, int ax, int64_t z0, int64_t z1) {
+  TilePlan P;
+  const int64_t nx = m->nx, ny = m->ny, nz = m->nz, S = m->S, es = sizeof(T);
+  const int64_t nzp = m->lod_dims == 2 ? 1 : nz;
+  const int n = axis_points(m, ax);
+  P.ch = closed_chunk(m, ax);
+  P.nc = (n + P.ch - 1) / P.ch;
+  const int W = P.w = P.ch == 32 && P.nc > 8 && (es == 8 || ax == 0) ? 16 : 32;
+  P.maxt = P.ch == 16 || W * P.nc > 256 ? 512 : 256;
+  if (W * P.nc > P.maxt) return P;
+  if (ax == 0) {
+    if (S > W) return P;
+    P.R = (int)(W / S);
+    const int64_t row = nx * S, rb = row * es;
+    const int mod = es == 8 ? 16 : 32;
+    int64_t pitch = row + ((S - row) % mod + mod) % mod;
+    if (rb % 16) {  // one copy of R rows
+      const int64_t g = rb % 8 ? 4 : 2;  // rows between 16-byte boundaries
+      P.R = (int)(P.R / g * g);
+      pitch = row;
+      if (P.R == 0 || (z1 >= 0 && (z0 * ny * rb) % 16)) return P;
+    } else {
+      while ((pitch * es) % 16) ++pitch;
+    }
+    if (P.R * S * 3 < W * 2) return P;  // too many lanes would repeat others' work
+    P.pitch = (int)pitch;
+    const int64_t rows = (z1 >= 0 ? (z1 - z0) : nzp) * ny;
+    P.ntiles = (uint32_t)((rows + P.R - 1) / P.R);
+    P.stage_elems = (int)((P.R * pitch + P.ch * S + 127) / 128 * 128);
+  } else {
+    const int64_t ls = ax == 1 ? nx * S : nx * ny * S, os = nx * ny * S * (ax == 1 ? 1 : nz);
+    const int64_t C = ls, outer = ax == 1 ? nzp : 1;
+    if ((ls * es) % 16 || (os * es) % 16 || C >= ((int64_t)1 << 31)) return P;
+    P.nboxes = (n + 255) / 256;
+    P.box_n = (n + P.nboxes - 1) / P.nboxes;
+    P.box_n += (P.box_n * W * es) % 128 ? 1 : 0;  // each box starts on a 128-byte boundary
+    const int64_t ct = (C + W - 1) / W;
+    P.ntiles = (uint32_t)(ct * outer);
+    if (z1 >= 0 && ax == 1) {
+      P.tile0 = (uint32_t)(ct * z0);
+      P.ntiles = (uint32_t)(ct * z1);
+    }
+    P.stage_elems = P.box_n * P.nboxes * W;
+  }
+  const size_t fold = 4 * (size_t)P.nc * W * sizeof(CT);  // two parities of U and W
+  const size_t stage = (size_t)P.stage_elems * es;
+  if (stage + fold + 1024 > kTileSmem) return P;
+  const int blocks =
+      std::max(1, bfvm::closed_min_blocks<CT>(P.ch, P.maxt) * P.maxt / (W * P.nc));
+  const size_t budget = std::max(kTileSmem / blocks - 1024, stage + fold);  // 1 KB: system, pad
+  P.stages = (int)std::min<size_t>(3, (budget - fold) / stage);
+  P.smem = P.stages * stage + fold + 128;
+  P.ok = true;
+  return P;
+}
+
+template <typename T, typename CT, int CH, int W, bool DIR, bool ROWS, int MAXT, bool EXACT>
+void tile_kernel(bfvm_solver* m, const CUtensorMap& map, const bfvm::ClosedTileArgs<T, CT>& a,
+                 dim3 block, size_t smem) {
+  auto k = bfvm::closed_tile_kernel<T, CT, CH, W, DIR, ROWS, MAXT, EXACT>;
+  allow_smem((const void*)k, m->device, smem);
+  int per_sm = 0;
+  BFVM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, block.x * block.y, smem));
+  require(per_sm > 0, "sweep kernel does not fit on an SM", BFVM_ERR_STATE);
+  const dim3 grid(std::min<uint32_t>(a.ntiles - a.tile0, (uint32_t)per_sm * m->num_sms));
+  k<<<grid, block, smem, m->stream>>>(map, a);
+  check_launch(m);
+}
+
+template <typename T, typename CT>
+void sweep_tiles(bfvm_solver* m, int ax, int fuse, int64_t z0, int64_t z1, const TilePlan& P) {
+  const int64_t nx = m->nx, ny = m->ny, nz = m->nz, S = m->S;
+  bfvm::ClosedTileArgs<T, CT> a{};
+  a.p = m->p.as<T>();
+  a.out = m->sweep_out ? static_cast<T*>(m->sweep_out) : m->p.as<T>();
+  a.tile0 = P.tile0;
+  a.ntiles = P.ntiles;
+  a.n = axis_points(m, ax);
+  a.S = (int)S;
+  a.mS = quot_of(S);
+  a.stages = P.stages;
+  a.stage_elems = P.stage_elems;
+  a.cc = closed_view<CT>(m, ax);
+  const DevSegList& dseg = ax == 0 ? m->seg_dir_x : m->seg_dir_y;
+  if (ax == 2 || !dseg.present) fuse = 0;
+  a.fuse = fuse & (bfvm::kFuseDirPro | bfvm::kFuseDirEpi);
+  a.dir = dseg.view();
+  a.status = m->d_status.as<int>();
+  if (ax == 0) {
+    a.row0 = z1 >= 0 ? z0 * ny : 0;
+    a.rows = z1 >= 0 ? z1 * ny : ny * (m->lod_dims == 2 ? 1 : nz);
+    a.R = P.R;
+    a.row_elems = (int)(nx * S);
+    a.pitch = P.pitch;
+  } else {
+    a.ls = ax == 1 ? nx * S : nx * ny * S;
+    a.os = nx * ny * S * (ax == 1 ? 1 : nz);
+    a.C = (uint32_t)a.ls;
+    a.ctiles = (a.C + P.w - 1) / P.w;
+    a.mT = quot_of(a.ctiles);
+    a.box_n = P.box_n;
+    a.nboxes = P.nboxes;
+    encode_lines_map(m, ax, sizeof(T), a.C, a.n, ax == 1 ? (m->lod_dims == 2 ? 1 : nz) : 1, a.ls,
+                     a.os, P.w, P.box_n);
+  }
+  const dim3 block(P.w, P.nc);
+  auto go = [&](auto ch, auto w, auto maxt) {
+    constexpr int CH = decltype(ch)::value, W = decltype(w)::value, MAXT = decltype(maxt)::value;
+    with_flags(
+        [&](auto dir, auto rows, auto exact) {
+          tile_kernel<T, CT, CH, W, decltype(dir)::value, decltype(rows)::value, MAXT,
+                      decltype(exact)::value>(m, m->maps[ax], a, block, P.smem);
+        },
+        a.fuse != 0, ax == 0, a.n % CH == 0);
+  };
+  using std::integral_constant;
+  if (P.ch == 16)
+    go(integral_constant<int, 16>(), integral_constant<int, 32>(), integral_constant<int, 512>());
+  else if (P.w == 32 && P.maxt == 256)
+    go(integral_constant<int, 32>(), integral_constant<int, 32>(), integral_constant<int, 256>());
+  else if (P.w == 32)
+    go(integral_constant<int, 32>(), integral_constant<int, 32>(), integral_constant<int, 512>());
+  else if (P.maxt == 256)
+    go(integral_constant<int, 32>(), integral_constant<int, 16>(), integral_constant<int, 256>());
+  else
+    go(integral_constant<int, 32>(), integral_constant<int, 16>(), integral_constant<int, 512>());
+}
+
+// Whether the tile kernel sweeps the axis rather than the line kernel (us, line
+// -> tile):
+//   x: 26.4 -> 22.9 at 128^3 x 4, 95.7 -> 79.3 at 192^3 x 4, 25.9 -> 22.4 at
+//     128^3 x 1, 460 either way at 256^3 x 10 (FP64), 1716 -> 1386 at 512^3 x
+//     8 FP32: rows arrive whole, where the line kernel's loads touch a few
+//     bytes of each sector.  At 16-point chunks only for one or two densities
+//     (30.2 -> 34.2 at 101^3 x 7).
+//   y and z: columns are contiguous and the line kernel, with more blocks per
+//     SM to hide its loads, is ahead (y 395 -> 458 at 256^3 x 10, FP32 1401 ->
+//     1837 at 512^3 x 8), except with an FP32 field in FP64 arithmetic (113 ->
+//     95 at 256^3 x 4: the conversions lengthen the solve), from 257 points
+//     on in FP64 (206 -> 189 at 400^3 x 1: one block per SM either way), and
+//     where 32-point chunks leave a partial one (FP32 70 -> 52 at 200^3 x 4).
+template <typename T, typename CT>
+bool tiles_better(const bfvm_solver* m, int ax, int ch) {
+  if (ax == 0) return ch == 32 || m->S <= 2;
+  if (ch == 16) return false;
+  const int n = axis_points(m, ax);
+  return sizeof(T) != sizeof(CT) || n % 32 != 0 || (sizeof(CT) == 8 && n > 256);
+}
+
+}  // namespace
+
+// One sweep of axis ax (planes [z0, z1) of the x and y axes, z1 < 0: all),
+// with the Dirichlet overwrites of `fuse` before and after it.
+void closed_sweep(bfvm_solver* m, int ax, int fuse, int64_t z0, int64_t z1) {
+  auto go = [&](auto t, auto ct) {
+    using T = decltype(t);
+    using CT = decltype(ct);
+    const TilePlan P = plan_tiles<T, CT>(m, ax, z0, z1);
+    if (P.ok && tiles_better<T, CT>(m, ax, P.ch))
+      sweep_tiles<T, CT>(m, ax, fuse, z0, z1, P);
+    else
+      sweep_lines<T, CT>(m, ax, fuse, z0, z1);
+  };
+  if (m->precision == BFVM_FP64)
+    go(double(), double());
+  else if (m->precision == BFVM_FP32_FP64MATH)
+    go(float(), double());
+  else
+    go(float(), float());
+}
+
+}  // namespace bfvm_rt

@@ -98,7 +98,7 @@ void choose_axes(bfvm_solver* m) {
 void clear_state_after_resize(bfvm_solver* m) {
   m->zs_ranks = 0;  // a z slab is declared again for the new mesh
   m->zs_bounds.clear();
-  m->p.ensure(std::max<size_t>(m->NS() * m->elem(), 16));
+  m->p.ensure(field_alloc(m->NS() * m->elem()));
   BFVM_CUDA(cudaMemsetAsync(m->p.ptr, 0, m->NS() * m->elem(), m->stream));
   m->setup_done = false;
   m->bulk_vox.clear();
@@ -209,6 +209,8 @@ void thomas_setup(bfvm_solver* m, double dt) {
   m->setup_dt = dt;
   m->setup_D = m->D;
   m->setup_decay = m->decay;
+  m->setup_dims = m->lod_dims;
+  closed_setup(m);
   m->setup_done = true;
 }
 
@@ -390,9 +392,17 @@ void build_bulk(bfvm_solver* m) {
   (void)S;
 }
 
+// Chunk length of the kernel that sweeps axis a (0 or 1) as things are set.
+int dir_chunk(const bfvm_solver* m, int a) {
+  return closed_axis(m, a) ? closed_axis_chunk(m, a) : m->axis[a].ch;
+}
+
 void build_dirichlet(bfvm_solver* m) {
-  if (!m->dir_dirty) return;
+  // the segments follow the chunk length of the kernel that reads them
+  if (!m->dir_dirty && m->dir_ch[0] == dir_chunk(m, 0) && m->dir_ch[1] == dir_chunk(m, 1)) return;
   ++m->lists_version;
+  m->dir_ch[0] = dir_chunk(m, 0);
+  m->dir_ch[1] = dir_chunk(m, 1);
   cudaStream_t st = m->stream;
   const int S = m->S;
   // Nodes are applied in list order, so for a repeated voxel the last one
@@ -419,7 +429,7 @@ void build_dirichlet(bfvm_solver* m) {
 
   // x sweep: lines are rows (k, j), points i
   {
-    const int ch = m->axis[0].ch, nc = (m->nx + ch - 1) / ch;
+    const int ch = m->dir_ch[0], nc = (m->nx + ch - 1) / ch;
     std::vector<int64_t> line(E);
     std::vector<int> pos(E);
     for (int64_t e = 0; e < E; ++e) {
@@ -433,7 +443,7 @@ void build_dirichlet(bfvm_solver* m) {
   }
   // y sweep: lines are (k, i), points j
   {
-    const int ch = m->axis[1].ch, nc = (m->ny + ch - 1) / ch;
+    const int ch = m->dir_ch[1], nc = (m->ny + ch - 1) / ch;
     std::vector<int64_t> key(E);
     for (int64_t e = 0; e < E; ++e) {
       const int64_t v = vox[e];
@@ -676,6 +686,26 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(ptr);
   }();
   return fn;
+}
+
+// The tensor map of axis ax as [nouter][n][C] (strides in elements) with
+// boxes of [box_n][w], encoded again when the field or its geometry changed.
+void encode_lines_map(bfvm_solver* m, int ax, int64_t es, int64_t C, int64_t n, int64_t nouter,
+                      int64_t ls, int64_t os, int w, int box_n) {
+  const int64_t geom[9] = {(int64_t)(uintptr_t)m->p.ptr, es, C, n, nouter, ls, os, w, box_n};
+  if (std::equal(geom, geom + 9, m->map_geom[ax])) return;
+  cuuint64_t dims[3] = {(cuuint64_t)C, (cuuint64_t)n, (cuuint64_t)nouter};
+  cuuint64_t strides[2] = {(cuuint64_t)(ls * es), (cuuint64_t)(os * es)};
+  cuuint32_t box[3] = {(cuuint32_t)w, (cuuint32_t)box_n, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = tensor_map_encoder()(
+      &m->maps[ax], es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+      3, m->p.ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  require(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")",
+          BFVM_ERR_CUDA);
+  std::copy(geom, geom + 9, m->map_geom[ax]);
 }
 
 // Raises the dynamic shared-memory limit of a kernel once per device (solvers
@@ -946,24 +976,7 @@ void launch_lines_st(const CUtensorMap& map, const bfvm::LinesArgs<T, CT>& a, in
 template <typename T, typename CT>
 void launch_lines(bfvm_solver* m, int ax, const LinesPlan& L, bool dir, int64_t z0 = 0,
                   int64_t z1 = -1) {
-  // (re)encode the tensor map when the field or its geometry changed
-  const int64_t es = (int64_t)sizeof(T);
-  const int64_t geom[9] = {(int64_t)(uintptr_t)m->p.ptr, es, L.C, L.n, L.nouter, L.ls, L.os,
-                           L.w, L.box_n};
-  if (!std::equal(geom, geom + 9, m->map_geom[ax])) {
-    cuuint64_t dims[3] = {(cuuint64_t)L.C, (cuuint64_t)L.n, (cuuint64_t)L.nouter};
-    cuuint64_t strides[2] = {(cuuint64_t)(L.ls * es), (cuuint64_t)(L.os * es)};
-    cuuint32_t box[3] = {(cuuint32_t)L.w, (cuuint32_t)L.box_n, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = tensor_map_encoder()(
-        &m->maps[ax], sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-        3, m->p.ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    require(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")",
-            BFVM_ERR_CUDA);
-    std::copy(geom, geom + 9, m->map_geom[ax]);
-  }
+  encode_lines_map(m, ax, sizeof(T), L.C, L.n, L.nouter, L.ls, L.os, L.w, L.box_n);
   bfvm::LinesArgs<T, CT> a{};
   a.p = m->p.as<T>();
   a.out = m->sweep_out ? static_cast<T*>(m->sweep_out) : a.p;
@@ -1268,6 +1281,10 @@ void sweep(bfvm_solver* m, int ax, int fuse, double dt, int64_t z0, int64_t z1) 
       long_sweep<double>(m, ax, fuse, z0, z1, dt);
     else
       long_sweep<float>(m, ax, fuse, z0, z1, dt);
+    return;
+  }
+  if (closed_axis(m, ax) && !(fuse & (bfvm::kFuseBulk | bfvm::kFuseCells))) {
+    closed_sweep(m, ax, fuse, z0, z1);
     return;
   }
   // under AUTO an axis may carry its own kernel choice (bfvm_tune_sweeps)
@@ -1592,6 +1609,7 @@ int bfvm_destroy(bfvm_solver* m) {
     m->d_status.release();
     m->d_grad.release();
     adjoint_release(m);
+    for (auto& c : m->closed_tab) c.release();
     for (auto& c : m->chunk) c.release();
     for (auto& c : m->chunk_il) c.release();
     for (auto& c : m->chunk_slots) c.release();
@@ -1694,7 +1712,7 @@ int bfvm_resize_densities(bfvm_solver* m, int num_densities) {
     m->D.assign(num_densities, 0.0);
     m->decay.assign(num_densities, 0.0);
     m->d_grad.release();
-    m->p.ensure(std::max<size_t>(m->NS() * m->elem(), 16));
+    m->p.ensure(field_alloc(m->NS() * m->elem()));
     BFVM_CUDA(cudaMemsetAsync(m->p.ptr, 0, m->NS() * m->elem(), m->stream));
     // resize_densities keeps the Dirichlet list but its value vectors no
     // longer match S; the list is cleared so no stale node is applied.
@@ -1718,7 +1736,7 @@ int bfvm_add_density(bfvm_solver* m, double diffusion_coefficient, double decay_
     const int S0 = m->S, S1 = S0 + 1;
     const int64_t N = m->N();
     DevBuf np;
-    np.ensure(std::max<size_t>((size_t)N * S1 * m->elem(), 16));
+    np.ensure(field_alloc((size_t)N * S1 * m->elem()));
     BFVM_CUDA(cudaMemsetAsync(np.ptr, 0, (size_t)N * S1 * m->elem(), m->stream));
     BFVM_CUDA(cudaMemcpy2DAsync(np.ptr, S1 * m->elem(), m->p.ptr, S0 * m->elem(),
                                 S0 * m->elem(), N, cudaMemcpyDeviceToDevice, m->stream));
@@ -2527,7 +2545,7 @@ int bfvm_set_precision(bfvm_solver* m, int precision) {
     if (was64 != is64) {  // the field changes element type
       const int64_t NS = m->NS();
       DevBuf np;
-      np.ensure(std::max<size_t>(NS * (is64 ? 8 : 4), 16));
+      np.ensure(field_alloc(NS * (is64 ? 8 : 4)));
       if (NS > 0) {
         if (!is64)
           bfvm::convert_kernel<float, double>
@@ -2686,18 +2704,9 @@ void tune_sweeps(bfvm_solver* m, double dt, int reps) {
         }
         if (nc <= 16) cand.push_back({BFVM_PATH_DIRECT, ch, 16, 0, 1, 0});
       }
-      Axis best = m->axis[ax];
       float best_ms = 1e30f;
-      for (const Choice& c : cand) {
-        Axis& A = m->axis[ax];
-        if (A.ch != c.ch) m->bulk_dirty = m->dir_dirty = m->ag_seg_dirty = true;
-        A.ch = c.ch;
-        A.tw = c.tw;
-        A.minb = c.minb;
-        A.kind = c.kind;
-        A.stages = c.stages;
-        A.build = c.build;
-        A.user = true;
+      Axis best;
+      auto trial = [&] {
         build_all(m);
         sweep(m, ax, fuses[ax], dt);  // warm-up: tables and plans
         BFVM_CUDA(cudaEventRecord(e0, m->stream));
@@ -2708,8 +2717,25 @@ void tune_sweeps(bfvm_solver* m, double dt, int reps) {
         BFVM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
         if (ms < best_ms) {
           best_ms = ms;
-          best = A;
+          best = m->axis[ax];
         }
+      };
+      // the default choice first (the closed-form kernels), then the others
+      m->axis[ax].user = false;
+      m->bulk_dirty = m->dir_dirty = m->ag_seg_dirty = true;
+      choose_axes(m);
+      trial();
+      for (const Choice& c : cand) {
+        Axis& A = m->axis[ax];
+        if (A.ch != c.ch) m->bulk_dirty = m->dir_dirty = m->ag_seg_dirty = true;
+        A.ch = c.ch;
+        A.tw = c.tw;
+        A.minb = c.minb;
+        A.kind = c.kind;
+        A.stages = c.stages;
+        A.build = c.build;
+        A.user = true;
+        trial();
       }
       if (m->axis[ax].ch != best.ch) m->bulk_dirty = m->dir_dirty = m->ag_seg_dirty = true;
       m->axis[ax] = best;

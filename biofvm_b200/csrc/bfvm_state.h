@@ -129,6 +129,10 @@ struct DeviceGuard {
   }
 };
 
+// Bytes allocated for a field: whole 16-byte words, which the bulk copies of
+// a field's last rows read to the end.
+inline size_t field_alloc(size_t bytes) { return std::max<size_t>((bytes + 15) / 16 * 16, 16); }
+
 inline int64_t blocks_for(int64_t work, int threads) { return (work + threads - 1) / threads; }
 
 }  // namespace bfvm_rt
@@ -168,6 +172,10 @@ struct bfvm_solver {
   int chunk_ch[3] = {0, 0, 0};
   int chunk_nslots[3] = {0, 0, 0};
   bfvm_rt::Axis axis[3];
+  // constants of the closed-form sweeps per axis (cst [S][8], pw [chunks][S][2]),
+  // built with the Thomas setup; lod_dims at that setup
+  bfvm_rt::DevBuf closed_tab[3];
+  int setup_dims = 3;
 
   // bulk sources/sinks: non-identity voxels, ascending
   std::vector<int64_t> bulk_vox;
@@ -189,6 +197,7 @@ struct bfvm_solver {
   std::vector<int64_t> dir_sorted;  // the unique nodes as uploaded (ascending)
   bfvm_rt::DevBuf d_dir_vox, d_dir_val;
   bfvm_rt::DevSegList seg_dir_x, seg_dir_y;
+  int dir_ch[2] = {0, 0};  // chunk lengths the x and y segments were built for
 
   // Agents, held on the device only: voxel[A], temp1[A][S], temp2[A][S] in
   // list order, and the list order stably sorted by voxel (key = voxel,
@@ -302,6 +311,14 @@ void bulk_any(bfvm_solver* m, double dt);
 void cells_any(bfvm_solver* m);
 template <typename T>
 void dirichlet_standalone(bfvm_solver* m);
+void encode_lines_map(bfvm_solver* m, int ax, int64_t es, int64_t C, int64_t n, int64_t nouter,
+                      int64_t ls, int64_t os, int w, int box_n);
+void allow_smem(const void* kernel, int device, size_t bytes);
+// Defined in bfvm_closed.cu.
+bool closed_axis(const bfvm_solver* m, int ax);
+int closed_axis_chunk(const bfvm_solver* m, int ax);
+void closed_setup(bfvm_solver* m);
+void closed_sweep(bfvm_solver* m, int ax, int fuse, int64_t z0, int64_t z1);
 // Defined in bfvm_adjoint.cu.
 void adjoint_release(bfvm_solver* m);
 

@@ -260,10 +260,11 @@ BFVM_API int bfvm_set_row_build(bfvm_solver* m, int build);
  * not apply, and before the first sweep has built the chunk tables). */
 BFVM_API int bfvm_get_row_build(bfvm_solver* m, int* requested, int* effective);
 /* Which sweep kernels run (all compute the same sweep):
- *   BFVM_PATH_AUTO    (default) the register kernel for x, the TMA-fed
- *                     persistent kernel for y and z where the layout allows
- *                     it (16-byte multiple row and plane strides), else
- *                     direct loads;
+ *   BFVM_PATH_AUTO    (default) the closed-form kernels (constant slopes, no
+ *                     per-point tables) on every axis of up to 1024 points
+ *                     whose kernel is not set by bfvm_set_sweep_config or
+ *                     the tuner, sources not fused into x; an axis set so
+ *                     runs the kernel it was set to;
  *   BFVM_PATH_GENERIC the first, table-free register kernel on every axis;
  *   BFVM_PATH_TMA     TMA-fed persistent kernels on every axis they fit;
  *   BFVM_PATH_DIRECT  direct-load kernels on every axis. */

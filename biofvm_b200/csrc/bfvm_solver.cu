@@ -2450,20 +2450,19 @@ int bfvm_compute_all_gradient_vectors(bfvm_solver* m) {
   return SOLVER_CALL(m, {
     ensure_gradients(m);
     // the reference divides by 2*dx, 2*dy, 2*dz (:704-713)
-    const double two_dx = m->dx * 2.0, two_dy = m->dy * 2.0, two_dz = m->dz * 2.0;
-    const int64_t work = m->NS();
-    const bool rows = m->ny <= 65535 && m->nz <= 65535 && (int64_t)m->nx * m->S < (1 << 30);
-    const dim3 rgrid((unsigned)blocks_for((int64_t)m->nx * m->S, 256), m->ny, m->nz);
+    const bfvm::Divisor dx{m->dx * 2.0, 0.5 / m->dx}, dy{m->dy * 2.0, 0.5 / m->dy},
+        dz{m->dz * 2.0, 0.5 / m->dz};
+    auto moderate = [](double d) { return d > 1e-20 && d < 1e20; };
+    const bool fast = moderate(m->dx) && moderate(m->dy) && moderate(m->dz);
+    const int64_t RS = (int64_t)m->nx * m->S;
+    const dim3 grid((unsigned)blocks_for(RS, 256),
+                    (unsigned)std::min<int64_t>(blocks_for(m->ny, bfvm::kGradRows), 65535),
+                    std::min(m->nz, 65535));
     with_types(m, [&](auto t, auto) {
       using T = decltype(t);
-      if (rows)
-        bfvm::gradient_rows_kernel<T><<<rgrid, 256, 0, m->stream>>>(
-            m->p.as<T>(), m->nx, m->ny, m->nz, m->S, two_dx, two_dy, two_dz,
-            m->d_grad.as<double>());
-      else
-        bfvm::gradient_kernel<T><<<(unsigned)blocks_for(work, 256), 256, 0, m->stream>>>(
-            m->p.as<T>(), m->nx, m->ny, m->nz, m->S, two_dx, two_dy, two_dz,
-            m->d_grad.as<double>());
+      auto k = fast ? bfvm::gradient_rows_kernel<T, true> : bfvm::gradient_rows_kernel<T, false>;
+      const bfvm::GradArgs a{RS, m->ny, m->nz, m->S, dx, dy, dz, m->d_grad.as<double>()};
+      k<<<grid, 256, 0, m->stream>>>(m->p.as<T>(), a);
     });
     check_launch(m);
   });

@@ -24,13 +24,14 @@ int axis_points(const bfvm_solver* m, int a) { return a == 0 ? m->nx : (a == 1 ?
 // us, at 256^3 x 4 FP32 132 -> 98), but a line's last, partial chunk runs the
 // body with bounds checks, a quarter of the threads of a 123-point line (z at
 // 161 x 97 x 123 x 3: 20.2 us at 16 points, 22.9 at 32).
+// Fields of few columns take 16 as well, to have threads on every SM (twelve
+// domains of 32 to 128 points a side, 20 steps: 4.19 -> 4.07 ms).
 int closed_chunk(const bfvm_solver* m, int a) {
   const int n = axis_points(m, a);
+  if (n > 512) return 32;
+  if (m->NS() / n * ((n + 31) / 32) < 128 * 148) return 16;
   return n % 32 == 0 || n > 160 ? 32 : 16;
 }
-
-// floor(2^64 / d) + 1 for quot(), 0 for d = 1.
-uint64_t quot_of(uint64_t d) { return d <= 1 ? 0 : ~(uint64_t)0 / d + 1; }
 
 }  // namespace
 
@@ -47,46 +48,52 @@ bool closed_axis(const bfvm_solver* m, int ax) {
 
 int closed_axis_chunk(const bfvm_solver* m, int ax) { return closed_chunk(m, ax); }
 
-// Constants of every axis from the coefficients of the Thomas setup
-// (BioFVM_solvers.cpp:105-126: c1 = dt D / dx^2, c2 = dt decay / 3, or / 2
-// for LOD_2D), in extended precision and rounded once.
-void closed_setup(bfvm_solver* m) {
-  const int S = m->S;
-  const double dt = m->setup_dt;
-  for (int a = 0; a < 3; ++a) {
-    const int n = axis_points(m, a);
-    if (n > 1024) continue;
-    const int ch = closed_chunk(m, a), nc = (n + ch - 1) / ch;
-    const bool fp32 = m->math_elem() == 4;
-    const size_t ncst = (size_t)S * 8, count = ncst + (size_t)nc * S * 2;
-    std::vector<double> t(count, 0.0);
-    std::vector<float> tf(fp32 ? 2 * count : 0, 0.0f);
-    for (int s = 0; s < S; ++s) {
-      const long double c1 = (long double)m->h_c1[a][s];
-      const long double c2 = (long double)m->setup_decay[s] * dt / (m->setup_dims == 2 ? 2 : 3);
-      // r = c1 / d with d the larger root of d^2 - (1 + 2 c1 + c2) d + c1^2
-      const long double b = 1 + 2 * c1 + c2;
-      const long double d = (b + std::sqrt((1 + c2) * (1 + c2 + 4 * c1))) / 2;
-      const long double r = fp32 ? (long double)(float)(c1 / d) : (long double)(double)(c1 / d);
-      auto put = [&](size_t i, long double x) {
-        t[i] = (double)x;
-        if (fp32) {
-          tf[2 * i] = (float)x;
-          tf[2 * i + 1] = (float)(x - tf[2 * i]);
-        }
-      };
-      auto power = [&](int k) { return std::pow(r, (long double)k); };
-      const int last = n - (nc - 1) * ch;
-      const long double k[7] = {r, (1 - r) * (1 - r) / (1 + c2), 1 / ((1 - r) * (1 + r)),
-                                power(ch), power(last), power(n), 1 / (1 - power(2 * n))};
-      for (int i = 0; i < 7; ++i) put((size_t)s * 8 + i, k[i]);
-      for (int c = 0; c < nc; ++c) {
-        const size_t i = ncst + ((size_t)c * S + s) * 2;
-        put(i, power(c * ch));
-        put(i + 1, power(n - std::min(n, (c + 1) * ch)));
+// Constants of axis a for ch-point chunks (ClosedCoef: cst, then pw) from the
+// coefficients of the Thomas setup (BioFVM_solvers.cpp:105-126: c1 = dt D /
+// dx^2, c2 = dt decay / 3, or / 2 for LOD_2D), in extended precision and
+// rounded once: to t, in FP32 to the pairs tf.
+void closed_constants(const bfvm_solver* m, int a, int ch, std::vector<double>& t,
+                      std::vector<float>& tf) {
+  const int S = m->S, n = axis_points(m, a), nc = (n + ch - 1) / ch;
+  const bool fp32 = m->math_elem() == 4;
+  const size_t ncst = (size_t)S * 8, count = ncst + (size_t)nc * S * 2;
+  t.assign(count, 0.0);
+  tf.assign(fp32 ? 2 * count : 0, 0.0f);
+  for (int s = 0; s < S; ++s) {
+    const long double c1 = (long double)m->h_c1[a][s];
+    const long double c2 =
+        (long double)m->setup_decay[s] * m->setup_dt / (m->setup_dims == 2 ? 2 : 3);
+    // r = c1 / d with d the larger root of d^2 - (1 + 2 c1 + c2) d + c1^2
+    const long double b = 1 + 2 * c1 + c2;
+    const long double d = (b + std::sqrt((1 + c2) * (1 + c2 + 4 * c1))) / 2;
+    const long double r = fp32 ? (long double)(float)(c1 / d) : (long double)(double)(c1 / d);
+    auto put = [&](size_t i, long double x) {
+      t[i] = (double)x;
+      if (fp32) {
+        tf[2 * i] = (float)x;
+        tf[2 * i + 1] = (float)(x - tf[2 * i]);
       }
+    };
+    auto power = [&](int k) { return std::pow(r, (long double)k); };
+    const int last = n - (nc - 1) * ch;
+    const long double k[7] = {r, (1 - r) * (1 - r) / (1 + c2), 1 / ((1 - r) * (1 + r)),
+                              power(ch), power(last), power(n), 1 / (1 - power(2 * n))};
+    for (int i = 0; i < 7; ++i) put((size_t)s * 8 + i, k[i]);
+    for (int c = 0; c < nc; ++c) {
+      const size_t i = ncst + ((size_t)c * S + s) * 2;
+      put(i, power(c * ch));
+      put(i + 1, power(n - std::min(n, (c + 1) * ch)));
     }
-    if (fp32)
+  }
+}
+
+void closed_setup(bfvm_solver* m) {
+  std::vector<double> t;
+  std::vector<float> tf;
+  for (int a = 0; a < 3; ++a) {
+    if (axis_points(m, a) > 1024) continue;
+    closed_constants(m, a, closed_chunk(m, a), t, tf);
+    if (m->math_elem() == 4)
       upload(m->closed_tab[a], tf, m->stream);
     else
       upload(m->closed_tab[a], t, m->stream);

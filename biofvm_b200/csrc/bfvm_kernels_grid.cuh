@@ -1,53 +1,73 @@
 // Whole steps of a small microenvironment in one cooperative launch.
 //
-// A field of up to ~1M voxel-densities with at most 64 points per axis costs
+// A field of up to 2^19 voxel-densities with at most 64 points per axis costs
 // more in kernel start-up than in work when every phase of a step is its own
-// launch (7 launches per step at 50^3 x 1).  Here every step runs inside one
-// launch over all SMs, as phases separated by grid-wide barriers of a
-// cooperative launch (all blocks are resident, so each barrier completes;
-// after the first step the sources ride on the z phase of the step before):
-//   sources: per bulk entry its update (BioFVM_microenvironment.cpp:603-609)
-//            and then its voxel's agents in list order
-//            (BioFVM_basic_agent.cpp:234-235); per agent voxel without a bulk
-//            entry its agents;
-//   x, y, z: tiles of TW lines x NC chunks of 4 or 8 points per block (as the
-//            register sweep kernel: chunk-local passes, the chunks' carries
-//            folded through shared memory, fix-ups); as a chunk is loaded, its
-//            Dirichlet nodes take their values (BioFVM_microenvironment.cpp:
-//            192-197, before each axis: BioFVM_solvers.cpp:177, 207, 241): a
-//            64-bit mask per line marks the nodes, whose values sit in a
-//            field-shaped array.
-// Every voxel lies on exactly one line per axis, so this equals the
-// reference's whole-field passes.  Lines are solved with the sweep kernels'
-// per-point tables (1/denominator, forward and backward slopes), within
-// 1e-12 of the reference's divisions.
+// launch.  Here every step runs inside one launch, as two phases separated by
+// grid-wide barriers of a cooperative launch (all blocks are resident, so each
+// barrier completes):
+//   xy: an item is one xy plane (of sg of its densities), held in shared
+//       memory.  As it is loaded, its voxels take the bulk update
+//       (BioFVM_microenvironment.cpp:603-609), then their agents in list order
+//       (BioFVM_basic_agent.cpp:234-235), then the Dirichlet values
+//       (BioFVM_microenvironment.cpp:192-197).  The x lines are solved in
+//       shared memory, the y lines from there to the field.  A node's value
+//       stays in its place through both: the x lines do not overwrite it, and
+//       the y lines pass it on, so that it is set before each axis
+//       (BioFVM_solvers.cpp:177, 207, 241).
+//   z:  tiles of columns, straight from and to the field.
+// Lines are solved as in bfvm_kernels_closed.cuh, in chunks of 8 points, one
+// per thread: sg is the most densities whose x lines and y lines are at most
+// one chunk per thread each.
+//
+// The steps are bound by latency: barriers, and the chains of a line.  A
+// grid barrier also empties L1, so that anything read again after it costs an
+// L2 round trip: the lines' constants are copied to shared memory once, and a
+// plane's loads are two rounds (the field with the maps, then what they point
+// to).  One block per SM: with two, the registers spill (50^3 x 4 22.7 ->
+// 32.7 us).  Steps of 50^3 x 1 with 1000 agents and a fixed boundary, 100 in a
+// call: 13.2 us, of three solvers at once 6.7 a step (16.9 and 9.9 with three
+// phases x, y, z through memory and the elimination's per-point tables); 24^3
+// x 20 14.1 (18.5), 32^3 x 8 12.9 (14.9), 64^3 x 2 16.1 (22.4), 50^3 x 4, with
+// more planes than SMs, 23.7 (22.5).
 #pragma once
 
 #include <cooperative_groups.h>
 
-#include "bfvm_kernels.cuh"
+#include "bfvm_kernels_closed.cuh"
 
 namespace bfvm {
+
+constexpr int kGridThreads = 512;
+constexpr int kGridChunk = 8;
+
+// what a voxel has (a byte each)
+enum : int { kVoxDirichlet = 1, kVoxBulk = 2, kVoxAgents = 4, kVoxMoreAgents = 8 };
 
 struct GridStepArgs {
   double* p;  // [nz][ny][nx][S]
   int nx, ny, nz, S;
   int nsteps;
   double dt;
-  bool bulk, cells;
-  // per axis: the sweep kernels' per-point tables [n][S] and c1 [S]
-  AxisCoef<double> coef[3];
-  // per voxel: its bulk entry and its first agent in the sorted list, or -1
+  int on;               // kVox* bits that take part
+  const double* cst[3]; // constants of the axes (ClosedCoef) for 8-point chunks
+  int cst_count[3];     // their lengths; copied to shared memory when staged
+  bool staged;
+  int sg, groups;       // densities per item, items per plane
+  int pitch;            // shared-memory elements between an item's rows
+  int tw;               // columns of a z tile: tw x chunks of nz <= kGridThreads
+  uint64_t m_sg, m_last, m_nx;  // quot() of sg, of the last item's, of nx,
+  uint64_t m_lx, m_ly, m_lx_last, m_ly_last, m_tw;  // of an item's x and y lines, of tw
+  const unsigned char* flags;   // [N]
+  // per flagged voxel: its bulk entry; its first agent's place in the sorted
+  // list and in the agent list
   const int* bulk_map;
-  const int* ag_map;
-  // Dirichlet nodes: per axis and line a mask of the points that are nodes
-  // (lines numbered x: k*ny + j, y: k*nx + i, z: j*nx + i), and the node
-  // values at their places in a field-shaped array [N][S]
-  bool dirichlet;
-  const unsigned long long* dir_mask[3];
+  const int2* ag_map;
+  // Dirichlet nodes: per x and y line a mask of the points that are nodes
+  // (lines numbered x: k*ny + j, y: k*nx + i), and the node values at their
+  // places in a field-shaped array [N][S]
+  const unsigned long long* dir_mask_x;
+  const unsigned long long* dir_mask_y;
   const double* dir_field;
-  int64_t nbulk;
-  const int64_t* bulk_vox;  // [E] ascending
   const double* bulk_st;    // [E][S] S*T
   const double* bulk_su;    // [E][S] U+S
   int64_t nagents;
@@ -57,235 +77,248 @@ struct GridStepArgs {
   const double* ag_t2;
 };
 
-// The agents of one voxel, from its first sorted entry r, in list order.
-__device__ __forceinline__ double grid_cells(const GridStepArgs& a, double x, int r, uint64_t vox,
-                                             int s) {
-  do {
-    const int64_t ai = __ldg(a.ag_idx + r);
-    x = cell_update(x, __ldg(a.ag_t1 + ai * a.S + s), __ldg(a.ag_t2 + ai * a.S + s));
-    ++r;
-  } while (r < a.nagents && __ldg(a.ag_key + r) == vox);
-  return x;
+// A chunk in registers through the block's fold: L columns, NC (at most 8)
+// chunks each, thread (col, c); threads without a chunk (c >= NC) only meet
+// the barrier.  cst: the axis's constants, in shared or global memory.
+__device__ __forceinline__ void grid_chunk(double (&v)[kGridChunk], int len, const double* cst,
+                                           int S, int s, double* sU, double* sW, int L, int NC,
+                                           int c, int col) {
+  const double2* k = reinterpret_cast<const double2*>(cst) + s * 4;
+  const double2 rs = k[0];
+  const double r = rs.x;
+  if (c < NC) closed_sums<double, kGridChunk, false>(v, len, r, sU[c * L + col], sW[c * L + col]);
+  __syncthreads();
+  if (c >= NC) return;
+  const double2 hrc = k[1], rlrn = k[2];
+  double u[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) u[i] = i < NC ? sU[i * L + col] : 0.0;
+  double TU = 0.0, q0 = 0.0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (i == c) q0 = TU;
+    if (i < NC) TU = fma(i == NC - 1 ? rlrn.x : hrc.y, TU, u[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) u[i] = i < NC ? sW[i * L + col] : 0.0;
+  double TW = 0.0, w0 = 0.0;
+#pragma unroll
+  for (int i = 7; i >= 0; --i) {
+    if (i == c) w0 = TW;
+    TW = fma(hrc.y, TW, u[i]);
+  }
+  const double2 pw = reinterpret_cast<const double2*>(cst + (size_t)S * 8)[c * S + s];
+  const double inv = k[3].x;
+  const double qin = fma(pw.x, fma(rlrn.y, TU, TW) * inv, q0);
+  const double vin = fma(pw.y, fma(rlrn.y, TW, TU) * inv, w0);
+  closed_solve<double, kGridChunk, false>(v, len, r, {rs.y, 0.0}, {hrc.x, 0.0}, qin, vin);
 }
 
-// Bulk then cell updates of every voxel that has either.
-__device__ __forceinline__ void grid_sources(const GridStepArgs& a, int64_t first,
-                                             int64_t stride) {
-  const int S = a.S;
-  const int64_t nb = a.bulk ? a.nbulk * S : 0;
-  const int64_t na = a.cells ? a.nagents * S : 0;
-  for (int64_t w = first; w < nb + na; w += stride) {
-    if (w < nb) {
-      const int64_t e = w / S;
-      const int s = (int)(w - e * S);
-      const int64_t vox = __ldg(a.bulk_vox + e);
-      double* q = a.p + vox * S + s;
-      double x = bulk_update(*q, __ldg(a.bulk_st + w), __ldg(a.bulk_su + w), a.dt);
-      if (a.cells) {
-        const int r = __ldg(a.ag_map + vox);
-        if (r >= 0) x = grid_cells(a, x, r, (uint64_t)vox, s);
+// A plane's values as the x sweep finds them, into shared memory: sources,
+// then Dirichlet values, a plane of up to 4096 in one round.  The field,
+// which other blocks wrote, is read past L1.
+__device__ __forceinline__ void grid_load(const GridStepArgs& a, int64_t vox0, int s0, int sg,
+                                          double* plane) {
+  constexpr int kMost = 8;
+  const int width = a.nx * sg, count = width * a.ny;
+  const uint64_t m_sg = sg == a.sg ? a.m_sg : a.m_last;
+  for (int first = threadIdx.x; first < count; first += kMost * kGridThreads) {
+    double x[kMost];
+    int f[kMost], be[kMost];
+    int2 ag[kMost];
+#pragma unroll
+    for (int q = 0; q < kMost; ++q) {
+      const int u = first + q * kGridThreads;
+      f[q] = 0;
+      if (u < count) {
+        const int vs = (int)quot(u, m_sg);  // voxel in the plane
+        const int64_t vox = vox0 + vs;
+        x[q] = __ldcg(a.p + vox * a.S + s0 + (u - vs * sg));
+        if (a.on) f[q] = __ldg(a.flags + vox);
+        if (a.on & kVoxBulk) be[q] = __ldg(a.bulk_map + vox);
+        if (a.on & kVoxAgents) ag[q] = __ldg(a.ag_map + vox);
       }
-      *q = x;
-    } else {
-      const int64_t r = (w - nb) / S;
-      const int s = (int)(w - nb - r * S);
-      const uint64_t vox = __ldg(a.ag_key + r);
-      if (r > 0 && __ldg(a.ag_key + r - 1) == vox) continue;  // not the voxel's first agent
-      if (a.bulk && __ldg(a.bulk_map + vox) >= 0) continue;   // done with its bulk entry
-      double* q = a.p + (int64_t)vox * S + s;
-      *q = grid_cells(a, *q, (int)r, vox, s);
+    }
+#pragma unroll
+    for (int q = 0; q < kMost; ++q) {
+      const int u = first + q * kGridThreads;
+      if (u < count) {
+        const int vs = (int)quot(u, m_sg), j = (int)quot(vs, a.m_nx);
+        const int64_t vox = vox0 + vs;
+        const int s = s0 + (u - vs * sg), flags = f[q] & a.on;
+        if (flags) {
+          if (flags & kVoxBulk) {
+            const int64_t e = (int64_t)be[q] * a.S + s;
+            x[q] = bulk_update(x[q], __ldg(a.bulk_st + e), __ldg(a.bulk_su + e), a.dt);
+          }
+          if (flags & kVoxAgents) {
+            int64_t e = (int64_t)ag[q].y * a.S + s;
+            x[q] = cell_update(x[q], __ldg(a.ag_t1 + e), __ldg(a.ag_t2 + e));
+            if (f[q] & kVoxMoreAgents) {
+              for (int r = ag[q].x + 1; r < a.nagents && __ldg(a.ag_key + r) == (uint64_t)vox;
+                   ++r) {
+                e = (int64_t)__ldg(a.ag_idx + r) * a.S + s;
+                x[q] = cell_update(x[q], __ldg(a.ag_t1 + e), __ldg(a.ag_t2 + e));
+              }
+            }
+          }
+          if (flags & kVoxDirichlet) x[q] = __ldg(a.dir_field + vox * a.S + s);
+        }
+        plane[j * a.pitch + (u - j * width)] = x[q];
+      }
     }
   }
 }
 
-// The lines of one axis in tiles of TW columns x NC chunks (TW = blockDim.x /
-// NC); columns are (line, density) pairs numbered as in lod_sweep_kernel.
-// sm holds 4 * blockDim.x values for the chunks' forward and backward carries.
-// With sources_after (z only), each stored point first takes the next step's
-// bulk and cell updates: every voxel lies on exactly one z chunk, so the
-// thread that solved it is the only one to touch it before the next x phase.
-template <int AX, int CH>
-__device__ __forceinline__ void grid_axis(const GridStepArgs& a, double* sm,
-                                          bool sources_after = false) {
-  const int S = a.S;
-  const int64_t plane = (int64_t)a.nx * a.ny;
-  const int n = AX == 0 ? a.nx : (AX == 1 ? a.ny : a.nz);
-  const int64_t C = AX == 0 ? S : (AX == 1 ? (int64_t)a.nx * S : plane * S);
-  const int64_t outer_stride = AX == 0 ? (int64_t)a.nx * S : (AX == 1 ? plane * S : 0);
-  const int64_t ls = AX == 0 ? S : (AX == 1 ? (int64_t)a.nx * S : plane * S);
-  const int64_t ncols = plane * a.nz / n * S;
-  const int NC = (n + CH - 1) / CH;
-  const int TW = blockDim.x / NC;
-  const int tx = threadIdx.x % TW;
-  const int c = threadIdx.x / TW;  // chunk; threads past NC chunks idle
-  const bool in_tile = c < NC;
-  const int k0 = c * CH;
-  double* sQ = sm;  // [NC][TW] forward chunk end values
-  double* sP = sQ + NC * TW;
-  double* sX = sP + NC * TW;  // backward chunk start values
-  double* sR = sX + NC * TW;
-  const AxisCoef<double> cf = a.coef[AX];
-  const int64_t ntiles = (ncols + TW - 1) / TW;
-  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t vcol = tile * TW + tx;
-    const bool active = in_tile && vcol < ncols;
-    const int len = active ? max(0, min(CH, n - k0)) : 0;
-    double* ptr = a.p;
-    const double* dptr = a.dir_field;
-    int s = 0;
-    unsigned long long nodes = 0ull;
-    if (active) {
-      const int64_t outer = vcol / C;
-      const int64_t col = vcol - outer * C;
-      const int64_t off = outer * outer_stride + col + (int64_t)k0 * ls;
-      ptr = a.p + off;
-      dptr = a.dir_field + off;
-      s = (int)(col % S);
-      if (a.dirichlet) nodes = __ldg(a.dir_mask[AX] + vcol / S) >> k0;
-    }
-    double v[CH];
+// One item of the xy phase.
+__device__ __forceinline__ void grid_xy(const GridStepArgs& a, int item, const double* cx,
+                                        const double* cy, double* plane, double* sU, double* sW) {
+  const int S = a.S, nx = a.nx, ny = a.ny;
+  const int k = item / a.groups, s0 = (item - k * a.groups) * a.sg;
+  const int sg = min(a.sg, S - s0);
+  const uint64_t m_sg = sg == a.sg ? a.m_sg : a.m_last;
+  const int64_t vox0 = (int64_t)k * nx * ny;
+  const int tid = threadIdx.x;
+  // x lines: columns (j, s), which meet distinct banks (pitch = sg mod 16);
+  // y lines: columns (i, s)
+  const int Lx = ny * sg, NCx = (nx + kGridChunk - 1) / kGridChunk;
+  const int Ly = nx * sg, NCy = (ny + kGridChunk - 1) / kGridChunk;
+  const int xc = (int)quot(tid, sg == a.sg ? a.m_lx : a.m_lx_last), xcol = tid - xc * Lx, xj = (int)quot(xcol, m_sg);
+  const int yc = (int)quot(tid, sg == a.sg ? a.m_ly : a.m_ly_last), ycol = tid - yc * Ly, yi = (int)quot(ycol, m_sg);
+  const int xlen = xc < NCx ? min(kGridChunk, nx - xc * kGridChunk) : 0;
+  const int ylen = yc < NCy ? min(kGridChunk, ny - yc * kGridChunk) : 0;
+  unsigned xnodes = 0, ynodes = 0;
+  if (a.on & kVoxDirichlet) {
+    if (xlen > 0)
+      xnodes = (unsigned)(__ldg(a.dir_mask_x + (int64_t)k * ny + xj) >> (xc * kGridChunk)) & 0xffu;
+    if (ylen > 0)
+      ynodes = (unsigned)(__ldg(a.dir_mask_y + (int64_t)k * nx + yi) >> (yc * kGridChunk)) & 0xffu;
+  }
+  grid_load(a, vox0, s0, sg, plane);
+  __syncthreads();
+  double v[kGridChunk];
+  {
+    const int s = xcol - xj * sg;
+    double* q = plane + xj * a.pitch + xc * kGridChunk * sg + s;
 #pragma unroll
-    for (int m = 0; m < CH; ++m)
-      v[m] = (m < len) ? (((nodes >> m) & 1ull) ? __ldg(dptr + m * ls) : ptr[m * ls]) : 0.0;
-    const double* c_inv = cf.inv_den + (int64_t)k0 * S + s;
-    const double* c_fwd = cf.fwd + (int64_t)k0 * S + s;
-    const double* c_bwd = cf.bwd + (int64_t)k0 * S + s;
-    // forward elimination, chunk-local with carry-in 0
-    const double c1 = active ? __ldg(cf.c1 + s) : 0.0;
-    double q = 0.0, P = 1.0;
+    for (int m = 0; m < kGridChunk; ++m) v[m] = m < xlen ? q[m * sg] : 0.0;
+    grid_chunk(v, xlen, cx, S, s0 + s, sU, sW, Lx, NCx, xc, xcol);
 #pragma unroll
-    for (int m = 0; m < CH; ++m) {
-      if (m < len) {
-        q = (v[m] + c1 * q) * __ldg(c_inv + m * S);
-        P = P * __ldg(c_fwd + m * S);
-        v[m] = q;
-      }
-    }
-    if (in_tile) {
-      sQ[c * TW + tx] = q;
-      sP[c * TW + tx] = P;
-    }
-    __syncthreads();
-    if (c > 0 && len > 0) {
-      double carry = 0.0;
-      for (int cc = 0; cc < c; ++cc) carry = sP[cc * TW + tx] * carry + sQ[cc * TW + tx];
-      double Pm = 1.0;
+    for (int m = 0; m < kGridChunk; ++m)
+      if (m < xlen && !(xnodes >> m & 1u)) q[m * sg] = v[m];
+  }
+  __syncthreads();
+  {
+    const int s = ycol - yi * sg;
+    const double* q = plane + yc * kGridChunk * a.pitch + ycol;
+    double* o = a.p + (vox0 + (int64_t)yc * kGridChunk * nx + yi) * S + s0 + s;
 #pragma unroll
-      for (int m = 0; m < CH; ++m) {
-        if (m < len) {
-          Pm = Pm * __ldg(c_fwd + m * S);
-          v[m] = v[m] + Pm * carry;
-        }
-      }
-    }
-    // back substitution, chunk-local with carry-in 0
-    double x = 0.0, R = 1.0;
+    for (int m = 0; m < kGridChunk; ++m) v[m] = m < ylen ? q[m * a.pitch] : 0.0;
+    grid_chunk(v, ylen, cy, S, s0 + s, sU, sW, Ly, NCy, yc, ycol);
 #pragma unroll
-    for (int m = CH - 1; m >= 0; --m) {
-      if (m < len) {
-        const double b = __ldg(c_bwd + m * S);
-        x = v[m] + b * x;
-        R = R * b;
-        v[m] = x;
-      }
-    }
-    if (in_tile) {
-      sX[c * TW + tx] = x;
-      sR[c * TW + tx] = R;
-    }
-    __syncthreads();
-    if (c < NC - 1 && len > 0) {
-      double carry = 0.0;
-      for (int cc = NC - 1; cc > c; --cc) carry = sR[cc * TW + tx] * carry + sX[cc * TW + tx];
-      double Rm = 1.0;
-#pragma unroll
-      for (int m = CH - 1; m >= 0; --m) {
-        if (m < len) {
-          Rm = Rm * __ldg(c_bwd + m * S);
-          v[m] = v[m] + Rm * carry;
-        }
-      }
-    }
-    if (AX == 2 && sources_after) {
-      const int64_t vox0 = vcol / S + (int64_t)k0 * plane;  // voxel of the chunk's point 0
-#pragma unroll
-      for (int m = 0; m < CH; ++m) {
-        if (m < len) {
-          const int64_t vox = vox0 + m * plane;
-          double x = v[m];
-          if (a.bulk) {
-            const int e = __ldg(a.bulk_map + vox);
-            if (e >= 0)
-              x = bulk_update(x, __ldg(a.bulk_st + (int64_t)e * S + s),
-                              __ldg(a.bulk_su + (int64_t)e * S + s), a.dt);
-          }
-          if (a.cells) {
-            const int r = __ldg(a.ag_map + vox);
-            if (r >= 0) x = grid_cells(a, x, r, (uint64_t)vox, s);
-          }
-          ptr[m * ls] = x;
-        }
-      }
-    } else {
-#pragma unroll
-      for (int m = 0; m < CH; ++m)
-        if (m < len) ptr[m * ls] = v[m];
-    }
-    __syncthreads();  // the carries of this tile are read before the next overwrites them
+    for (int m = 0; m < kGridChunk; ++m)
+      if (m < ylen) o[(int64_t)m * nx * S] = ynodes >> m & 1u ? q[m * a.pitch] : v[m];
   }
 }
 
-// nsteps whole steps with CH-point chunks (4 or 8: lines of <= 64 points in
-// at most 16 or 8 chunks); launched cooperatively (every block resident) with
-// 4 * blockDim.x doubles of dynamic shared memory.
-template <int CH>
-__global__ void __launch_bounds__(128) grid_steps_kernel(const GridStepArgs a) {
+// One tile of the z phase: TW columns.
+__device__ __forceinline__ void grid_z(const GridStepArgs& a, int tile, int TW, const double* cz,
+                                       double* sU, double* sW) {
+  const int S = a.S, ncols = a.nx * a.ny * S;
+  const int NC = (a.nz + kGridChunk - 1) / kGridChunk;
+  const int c = (int)quot(threadIdx.x, a.m_tw), tx = threadIdx.x - c * TW;
+  const int col = tile * TW + tx;
+  const int len = c < NC && col < ncols ? min(kGridChunk, a.nz - c * kGridChunk) : 0;
+  const int s = min(col, ncols - 1) % S;
+  double* q = a.p + (int64_t)c * kGridChunk * ncols + col;
+  double v[kGridChunk];
+#pragma unroll
+  for (int m = 0; m < kGridChunk; ++m) v[m] = m < len ? __ldcg(q + (int64_t)m * ncols) : 0.0;
+  grid_chunk(v, len, cz, S, s, sU, sW, TW, NC, c, tx);
+#pragma unroll
+  for (int m = 0; m < kGridChunk; ++m)
+    if (m < len) q[(int64_t)m * ncols] = v[m];
+}
+
+// Doubles of dynamic shared memory before the staged constants: the fold's
+// two sums, and the plane.
+__host__ __device__ constexpr int grid_smem_doubles(int ny, int pitch) {
+  return (2 * kGridThreads + ny * pitch + 1) / 2 * 2;
+}
+
+// nsteps whole steps; launched cooperatively (every block resident).
+static __global__ void __launch_bounds__(kGridThreads, 1) grid_steps_kernel(const GridStepArgs a) {
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
-  extern __shared__ double grid_carries[];
-  const int first = blockIdx.x * blockDim.x + threadIdx.x;
-  const int stride = gridDim.x * blockDim.x;
-  const bool sources = a.bulk || a.cells;
-  for (int step = 0; step < a.nsteps; ++step) {
-    // the first step's sources get a phase of their own; later steps' were
-    // applied as the previous z phase stored its lines
-    if (sources && step == 0) {
-      grid_sources(a, first, stride);
-      grid.sync();
+  extern __shared__ __align__(16) double grid_smem[];
+  double* sU = grid_smem;
+  double* sW = sU + kGridThreads;
+  double* plane = sW + kGridThreads;
+  const double* cst[3] = {a.cst[0], a.cst[1], a.cst[2]};
+  if (a.staged) {
+    double* t = grid_smem + grid_smem_doubles(a.ny, a.pitch);
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+      for (int i = threadIdx.x; i < a.cst_count[ax]; i += kGridThreads) t[i] = __ldg(cst[ax] + i);
+      cst[ax] = t;
+      t += a.cst_count[ax];  // an even number
     }
-    grid_axis<0, CH>(a, grid_carries);
+  }
+  const int items = a.nz * a.groups;
+  const int TW = a.tw;
+  const int tiles = (a.nx * a.ny * a.S + TW - 1) / TW;
+  for (int step = 0; step < a.nsteps; ++step) {
+    // (the barrier after a plane's load also completes the staging above)
+    for (int i = blockIdx.x; i < items; i += gridDim.x) {
+      grid_xy(a, i, cst[0], cst[1], plane, sU, sW);
+      __syncthreads();  // the fold and the plane are free again
+    }
     grid.sync();
-    grid_axis<1, CH>(a, grid_carries);
-    grid.sync();
-    grid_axis<2, CH>(a, grid_carries, sources && step + 1 < a.nsteps);
-    grid.sync();
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+      grid_z(a, t, TW, cst[2], sU, sW);
+      __syncthreads();
+    }
+    if (step + 1 < a.nsteps) grid.sync();
   }
 }
 
 // Dense voxel maps of the bulk entries and of the first agent of each voxel
-// in the sorted list (both -1 beforehand), and the Dirichlet nodes' line
-// masks (0 beforehand) and values at their places in the field.
-static __global__ void grid_maps_kernel(int* __restrict__ bulk_map, int* __restrict__ ag_map,
-                                        int64_t nbulk, const int64_t* __restrict__ bulk_vox,
-                                        int64_t nagents, const uint64_t* __restrict__ ag_key,
-                                        int64_t ndir, const int64_t* __restrict__ dir_vox,
+// in the sorted list, the voxels' flags, and the Dirichlet nodes' line masks
+// (flags and masks 0 beforehand) and values at their places in the field.
+// Entries of the maps that no flag points to are not written.
+static __global__ void grid_maps_kernel(int* __restrict__ bulk_map, int2* __restrict__ ag_map,
+                                        unsigned* __restrict__ flag_words, int64_t nbulk,
+                                        const int64_t* __restrict__ bulk_vox, int64_t nagents,
+                                        const uint64_t* __restrict__ ag_key,
+                                        const int* __restrict__ ag_idx, int64_t ndir,
+                                        const int64_t* __restrict__ dir_vox,
                                         const double* __restrict__ dir_val,
                                         unsigned long long* __restrict__ mx,
                                         unsigned long long* __restrict__ my,
-                                        unsigned long long* __restrict__ mz,
                                         double* __restrict__ dir_field, int nx, int ny, int S) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  auto flag = [&](int64_t v, int bits) {
+    atomicOr(flag_words + (v >> 2), (unsigned)bits << (8 * (v & 3)));
+  };
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
        i < nbulk || i < nagents || i < ndir; i += stride) {
-    if (i < nbulk) bulk_map[bulk_vox[i]] = (int)i;
-    if (i < nagents && (i == 0 || ag_key[i] != ag_key[i - 1])) ag_map[ag_key[i]] = (int)i;
+    if (i < nbulk) {
+      bulk_map[bulk_vox[i]] = (int)i;
+      flag(bulk_vox[i], kVoxBulk);
+    }
+    if (i < nagents && (i == 0 || ag_key[i] != ag_key[i - 1])) {
+      const uint64_t v = ag_key[i];
+      ag_map[v] = make_int2((int)i, ag_idx[i]);
+      flag((int64_t)v,
+           i + 1 < nagents && ag_key[i + 1] == v ? kVoxAgents | kVoxMoreAgents : kVoxAgents);
+    }
     if (i < ndir) {
       const int64_t v = dir_vox[i];
       const int64_t plane = (int64_t)nx * ny;
       const int64_t k = v / plane, ij = v - k * plane, j = ij / nx, ii = ij - j * nx;
-      atomicOr(mx + v / nx, 1ull << ii);
+      flag(v, kVoxDirichlet);
+      atomicOr(mx + k * ny + j, 1ull << ii);
       atomicOr(my + k * nx + ii, 1ull << j);
-      atomicOr(mz + ij, 1ull << k);
       for (int s = 0; s < S; ++s) dir_field[v * S + s] = dir_val[i * S + s];
     }
   }

@@ -211,6 +211,7 @@ void thomas_setup(bfvm_solver* m, double dt) {
   m->setup_decay = m->decay;
   m->setup_dims = m->lod_dims;
   closed_setup(m);
+  m->grid_tab_ok = false;
   m->setup_done = true;
 }
 
@@ -1615,6 +1616,7 @@ int bfvm_destroy(bfvm_solver* m) {
     for (auto& c : m->chunk_slots) c.release();
     for (auto& c : m->cl_tab) c.release();
     m->d_grid_maps.release();
+    for (auto& c : m->grid_tab) c.release();
     cudaStreamDestroy(m->stream);
     delete m;
   });
@@ -2243,103 +2245,118 @@ void cluster_run(bfvm_solver* m, double dt, int nsteps, int flags, int cl) {
   check_launch(m);
 }
 
-constexpr int kGridMaxN = 64;              // points per axis (registers per line)
-// voxel-densities: measured faster than the sweep kernels up to 2^19 (18.7 vs
-// 26.7 us/step at 50^3 x 1, 24.8 vs 27.2 at 50^3 x 4), even at 2^20
+constexpr int kGridMaxN = 64;  // points per axis (8-point chunks, 8 of them)
+// voxel-densities: at 64^3 x 2 = 2^19 16.1 us a step against 40 with the
+// sweep kernels, at 50^3 x 4 23.7 against 28.7
 constexpr int64_t kGridMaxVS = 1 << 19;
-constexpr int kGridThreads = 128;
-constexpr size_t kGridSmem = (size_t)4 * kGridThreads * sizeof(double);  // chunk carries
 
-// Tiles of the widest phase of grid steps with ch-point chunks (TW = threads
-// / chunks columns per tile).
-int64_t grid_tiles(const bfvm_solver* m, int ch) {
-  const int64_t N = (int64_t)m->nx * m->ny * m->nz;
-  const int ns[3] = {m->nx, m->ny, m->nz};
-  int64_t tiles = 1;
-  for (int ax = 0; ax < 3; ++ax) {
-    const int nc = (ns[ax] + ch - 1) / ch;
-    const int64_t tw = kGridThreads / nc;
-    tiles = std::max(tiles, (N / ns[ax] * m->S + tw - 1) / tw);
-  }
-  return tiles;
+constexpr size_t kGridSmemMost = 200 * 1024;
+
+// Doubles of an axis's constants at the grid steps' chunks.
+size_t grid_constants(int n, int S) {
+  return (size_t)S * (8 + 2 * ((n + bfvm::kGridChunk - 1) / bfvm::kGridChunk));
 }
 
-// Blocks of the cooperative launch that runs this solver's steps in one
-// launch, or 0 when bfvm_step uses the sweep kernels (or the cluster).  *ch:
-// the chunk length, 4 when the widest phase fits one wave of resident blocks
-// (shorter chains, measured faster: 50^3 x 1 19.9 -> 17.8 us/step, 32^3 x 8
-// 21.5 -> 16.8), else 8 (50^3 x 4: 27.3 us/step, 33.4 with 4-point chunks in
-// two waves).
-int grid_blocks(bfvm_solver* m, int* ch = nullptr) {
+struct GridPlan {
+  int blocks = 0;  // 0: bfvm_step does not take the grid steps
+  int sg = 0, groups = 0, pitch = 0;
+  int tw = 0;
+  bool staged = false;  // the lines' constants in shared memory
+  size_t smem = 0;
+};
+
+// The cooperative launch that runs this solver's steps in one launch.
+GridPlan plan_grid(bfvm_solver* m) {
+  GridPlan P;
   if (!m->grid_steps || m->path != BFVM_PATH_AUTO || m->precision != BFVM_FP64 ||
-      m->lod_dims != 3 || !m->uniform || m->fuse_sources || m->slab_planes > 0)
-    return 0;
-  if (m->nx > kGridMaxN || m->ny > kGridMaxN || m->nz > kGridMaxN) return 0;
-  if ((int64_t)m->NS() > kGridMaxVS || cluster_blocks(m) > 0) return 0;
-  if (m->grid_per_sm[0] == 0) {
-    int coop = 0;
+      m->lod_dims != 3 || !m->uniform || m->fuse_sources || m->slab_planes > 0 || m->zs_ranks > 0)
+    return P;
+  if (m->nx > kGridMaxN || m->ny > kGridMaxN || m->nz > kGridMaxN) return P;
+  if ((int64_t)m->NS() > kGridMaxVS || cluster_blocks(m) > 0) return P;
+  const int cx = (m->nx + bfvm::kGridChunk - 1) / bfvm::kGridChunk;
+  const int cy = (m->ny + bfvm::kGridChunk - 1) / bfvm::kGridChunk;
+  // densities per item: as many as the block's threads hold, fewer while that
+  // spreads the planes over more SMs
+  P.sg = std::max(1, std::min(m->S, bfvm::kGridThreads / std::max(m->ny * cx, m->nx * cy)));
+  P.groups = std::max((m->S + P.sg - 1) / P.sg, std::min(m->S, m->num_sms / m->nz));
+  P.sg = (m->S + P.groups - 1) / P.groups;
+  P.groups = (m->S + P.sg - 1) / P.sg;
+  const int width = m->nx * P.sg;
+  P.pitch = width + ((P.sg - width) % 16 + 16) % 16;
+  size_t doubles = bfvm::grid_smem_doubles(m->ny, P.pitch);
+  size_t consts = 0;
+  for (int n : {m->nx, m->ny, m->nz}) consts += grid_constants(n, m->S);
+  P.staged = (doubles + consts) * sizeof(double) <= kGridSmemMost;
+  if (P.staged) doubles += consts;
+  P.smem = doubles * sizeof(double);
+  // columns per z tile: whole warps, no more tiles than planes (or 32) need,
+  // so that other solvers' launches find SMs
+  const int64_t cols = (int64_t)m->nx * m->ny * m->S;
+  const int cz = (m->nz + bfvm::kGridChunk - 1) / bfvm::kGridChunk;
+  const int64_t tiles = 32 * std::max<int64_t>((int64_t)m->nz * P.groups, 32);
+  P.tw = (int)std::min<int64_t>(bfvm::kGridThreads / cz / 32 * 32, (cols + tiles - 1) / tiles * 32);
+  const int64_t work = std::max<int64_t>((int64_t)m->nz * P.groups, blocks_for(cols, P.tw));
+  if (m->grid_smem != P.smem) {
+    const void* k = (const void*)bfvm::grid_steps_kernel;
+    int coop = 0, per_sm = 0;
     BFVM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->device));
-    int per4 = 0, per8 = 0;
     if (coop) {
-      allow_smem((const void*)bfvm::grid_steps_kernel<4>, m->device, kGridSmem);
-      allow_smem((const void*)bfvm::grid_steps_kernel<8>, m->device, kGridSmem);
-      BFVM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per4, bfvm::grid_steps_kernel<4>, kGridThreads, kGridSmem));
-      BFVM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per8, bfvm::grid_steps_kernel<8>, kGridThreads, kGridSmem));
+      allow_smem(k, m->device, P.smem);
+      BFVM_CUDA(
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, bfvm::kGridThreads, P.smem));
     }
-    m->grid_per_sm[0] = per4 > 0 ? per4 : -1;
-    m->grid_per_sm[1] = per8 > 0 ? per8 : -1;
+    m->grid_resident = std::min(per_sm, 1) * m->num_sms;
+    m->grid_smem = P.smem;
   }
-  const int64_t sources =
-      (((int64_t)m->bulk_vox.size() + m->n_agents) * m->S + kGridThreads - 1) / kGridThreads;
-  for (int i = 0; i < 2; ++i) {
-    const int c = i == 0 ? 4 : 8;
-    if (m->grid_per_sm[i] < 0) continue;
-    const int64_t wave = (int64_t)m->grid_per_sm[i] * m->num_sms;
-    const int64_t tiles = grid_tiles(m, c);
-    if (tiles <= wave || c == 8) {
-      if (ch) *ch = c;
-      return (int)std::min<int64_t>(std::max(tiles, sources), wave);
-    }
-  }
-  return 0;
+  P.blocks = (int)std::min<int64_t>(work, m->grid_resident);
+  return P;
 }
 
 // nsteps whole steps (bulk -> cells -> LOD_3D) in one cooperative launch.
-void grid_run(bfvm_solver* m, double dt, int nsteps, int flags, int blocks, int ch) {
+void grid_run(bfvm_solver* m, double dt, int nsteps, int flags, const GridPlan& P) {
   const int S = m->S;
-  // scratch: Dirichlet values [N][S] (doubles first), line masks of the x, y
-  // and z lines, bulk and agent maps [N] each
+  if (!m->grid_tab_ok) {
+    std::vector<double> t;
+    std::vector<float> tf;
+    for (int a = 0; a < 3; ++a) {
+      closed_constants(m, a, bfvm::kGridChunk, t, tf);
+      upload(m->grid_tab[a], t, m->stream);
+    }
+    m->grid_tab_ok = true;
+  }
+  // scratch: Dirichlet values [N][S] (doubles first), line masks of the x and
+  // y lines, voxel flags, agent and bulk maps [N]
   const int64_t N = m->N();
-  const int64_t lx = N / m->nx, ly = N / m->ny, lz = N / m->nz;
+  const int64_t lx = N / m->nx, ly = N / m->ny;
   const size_t field_b = (size_t)N * S * sizeof(double);
-  const size_t masks_b = (size_t)(lx + ly + lz) * sizeof(uint64_t);
+  const size_t masks_b = (size_t)(lx + ly) * sizeof(uint64_t);
+  const size_t flags_b = ((size_t)N + 15) / 16 * 16;
   const void* before = m->d_grid_maps.ptr;
-  m->d_grid_maps.ensure(field_b + masks_b + (size_t)2 * N * sizeof(int));
+  m->d_grid_maps.ensure(field_b + masks_b + flags_b + (size_t)3 * N * sizeof(int));
   unsigned char* base = m->d_grid_maps.as<unsigned char>();
   double* dir_field = reinterpret_cast<double*>(base);
   unsigned long long* mx = reinterpret_cast<unsigned long long*>(base + field_b);
   unsigned long long* my = mx + lx;
-  unsigned long long* mz = my + ly;
-  int* maps = reinterpret_cast<int*>(base + field_b + masks_b);
+  unsigned char* vox_flags = base + field_b + masks_b;
+  int2* ag_map = reinterpret_cast<int2*>(vox_flags + flags_b);
+  int* bulk_map = reinterpret_cast<int*>(ag_map + N);
   const int64_t nbulk = (int64_t)m->bulk_vox.size();
   // the maps are rebuilt only when a list changed since they were built (or
   // the buffer moved, or the number of densities changed)
   const bool rebuild = m->grid_maps_version != m->lists_version || before != m->d_grid_maps.ptr ||
                        m->grid_maps_S != S;
   if (rebuild) {
-    BFVM_CUDA(cudaMemsetAsync(mx, 0, masks_b, m->stream));
-    BFVM_CUDA(cudaMemsetAsync(maps, 0xFF, (size_t)2 * N * sizeof(int), m->stream));
+    BFVM_CUDA(cudaMemsetAsync(mx, 0, masks_b + flags_b, m->stream));
     m->grid_maps_version = m->lists_version;
     m->grid_maps_S = S;
   }
   const int64_t most = std::max({nbulk, m->n_agents, m->dir_unique});
   if (rebuild && most > 0) {
     bfvm::grid_maps_kernel<<<(unsigned)blocks_for(most, 256), 256, 0, m->stream>>>(
-        maps, maps + N, nbulk, m->d_bulk_vox.as<int64_t>(), m->n_agents,
-        m->d_ag_key.as<uint64_t>(), m->dir_unique, m->d_dir_vox.as<int64_t>(),
-        m->d_dir_val.as<double>(), mx, my, mz, dir_field, m->nx, m->ny, S);
+        bulk_map, ag_map, reinterpret_cast<unsigned*>(vox_flags), nbulk,
+        m->d_bulk_vox.as<int64_t>(), m->n_agents, m->d_ag_key.as<uint64_t>(), m->d_ag_idx.as<int>(),
+        m->dir_unique, m->d_dir_vox.as<int64_t>(), m->d_dir_val.as<double>(), mx, my, dir_field,
+        m->nx, m->ny, S);
     check_launch(m);
   }
   bfvm::GridStepArgs a{};
@@ -2350,18 +2367,34 @@ void grid_run(bfvm_solver* m, double dt, int nsteps, int flags, int blocks, int 
   a.S = S;
   a.nsteps = nsteps;
   a.dt = dt;
-  a.bulk = (flags & BFVM_STEP_BULK) && nbulk > 0;
-  a.cells = (flags & BFVM_STEP_CELLS) && m->n_agents > 0;
-  for (int ax = 0; ax < 3; ++ax) a.coef[ax] = coef_view<double>(m, ax);
-  a.bulk_map = maps;
-  a.ag_map = maps + N;
-  a.dirichlet = m->dir_unique > 0;
-  a.dir_mask[0] = mx;
-  a.dir_mask[1] = my;
-  a.dir_mask[2] = mz;
+  if ((flags & BFVM_STEP_BULK) && nbulk > 0) a.on |= bfvm::kVoxBulk;
+  if ((flags & BFVM_STEP_CELLS) && m->n_agents > 0) a.on |= bfvm::kVoxAgents;
+  if (m->dir_unique > 0) a.on |= bfvm::kVoxDirichlet;
+  const int ns[3] = {m->nx, m->ny, m->nz};
+  for (int ax = 0; ax < 3; ++ax) {
+    a.cst[ax] = m->grid_tab[ax].as<double>();
+    a.cst_count[ax] = (int)grid_constants(ns[ax], S);
+  }
+  a.staged = P.staged;
+  a.sg = P.sg;
+  a.groups = P.groups;
+  a.pitch = P.pitch;
+  a.tw = P.tw;
+  a.m_sg = quot_of(P.sg);
+  a.m_nx = quot_of(m->nx);
+  const int last = S - (P.groups - 1) * P.sg;
+  a.m_last = quot_of(last);
+  a.m_lx = quot_of((uint64_t)m->ny * P.sg);
+  a.m_ly = quot_of((uint64_t)m->nx * P.sg);
+  a.m_lx_last = quot_of((uint64_t)m->ny * last);
+  a.m_ly_last = quot_of((uint64_t)m->nx * last);
+  a.m_tw = quot_of(P.tw);
+  a.flags = vox_flags;
+  a.bulk_map = bulk_map;
+  a.ag_map = ag_map;
+  a.dir_mask_x = mx;
+  a.dir_mask_y = my;
   a.dir_field = dir_field;
-  a.nbulk = nbulk;
-  a.bulk_vox = m->d_bulk_vox.as<int64_t>();
   a.bulk_st = m->d_bulk_st.as<double>();
   a.bulk_su = m->d_bulk_su.as<double>();
   a.nagents = m->n_agents;
@@ -2370,10 +2403,8 @@ void grid_run(bfvm_solver* m, double dt, int nsteps, int flags, int blocks, int 
   a.ag_t1 = m->d_ag_t1.as<double>();
   a.ag_t2 = m->d_ag_t2.as<double>();
   void* params[] = {&a};
-  const void* k = ch == 4 ? (const void*)bfvm::grid_steps_kernel<4>
-                          : (const void*)bfvm::grid_steps_kernel<8>;
-  BFVM_CUDA(cudaLaunchCooperativeKernel(k, dim3((unsigned)blocks), dim3(kGridThreads), params,
-                                        kGridSmem, m->stream));
+  BFVM_CUDA(cudaLaunchCooperativeKernel((const void*)bfvm::grid_steps_kernel, dim3((unsigned)P.blocks),
+                                        dim3(bfvm::kGridThreads), params, P.smem, m->stream));
   check_launch(m);
 }
 
@@ -2386,7 +2417,7 @@ int bfvm_set_grid_steps(bfvm_solver* m, int enable) {
 int bfvm_get_grid_steps(bfvm_solver* m, int* blocks) {
   return SOLVER_CALL(m, {
     require(blocks != nullptr, "null output pointer");
-    *blocks = grid_blocks(m);
+    *blocks = plan_grid(m).blocks;
   });
 }
 
@@ -2426,13 +2457,12 @@ int bfvm_step(bfvm_solver* m, double dt, int nsteps, int flags) {
       cluster_run(m, dt, nsteps, flags, cl);
       return;
     }
-    int gch = 8;
-    const int gb = nsteps > 0 ? grid_blocks(m, &gch) : 0;
-    if (gb > 0) {
+    const GridPlan grid = nsteps > 0 ? plan_grid(m) : GridPlan();
+    if (grid.blocks > 0) {
       check_lod_mesh(m);
       if (!m->setup_done) thomas_setup(m, dt);
       build_all(m);
-      grid_run(m, dt, nsteps, flags, gb, gch);
+      grid_run(m, dt, nsteps, flags, grid);
       return;
     }
     for (int it = 0; it < nsteps; ++it) step_once(m, dt, flags, nullptr);

@@ -133,6 +133,9 @@ struct DeviceGuard {
 // a field's last rows read to the end.
 inline size_t field_alloc(size_t bytes) { return std::max<size_t>((bytes + 15) / 16 * 16, 16); }
 
+// floor(2^64 / d) + 1 for the kernels' quot(), 0 for d = 1.
+inline uint64_t quot_of(uint64_t d) { return d <= 1 ? 0 : ~(uint64_t)0 / d + 1; }
+
 inline int64_t blocks_for(int64_t work, int threads) { return (work + threads - 1) / threads; }
 
 }  // namespace bfvm_rt
@@ -238,8 +241,7 @@ struct bfvm_solver {
   bfvm_rt::DevBuf cl_tab[3];
   // whole steps of a small field in one cooperative launch over all SMs
   // (bfvm_step under BFVM_PATH_AUTO, on by default): enabled flag, the per-call
-  // scratch (Dirichlet values and line masks, bulk and agent voxel maps), and
-  // the kernels' resident blocks per SM (0: not queried yet)
+  // scratch (Dirichlet values and line masks, bulk and agent voxel maps)
   int grid_steps = 1;
   bfvm_rt::DevBuf d_grid_maps;
   // the device lists change: every rebuild of the bulk, Dirichlet or agent
@@ -247,7 +249,12 @@ struct bfvm_solver {
   int64_t lists_version = 0;
   int64_t grid_maps_version = -1;
   int grid_maps_S = 0;
-  int grid_per_sm[2] = {0, 0};  // 4- and 8-point chunk kernels (-1: not usable)
+  // constants of the three axes for the grid steps' 8-point chunks, rebuilt
+  // after each Thomas setup
+  bool grid_tab_ok = false;
+  int grid_resident = 0;  // blocks of the grid steps the device holds at grid_smem
+  size_t grid_smem = 0;
+  bfvm_rt::DevBuf grid_tab[3];
   // cached tensor maps of the line sweeps, per axis, with the geometry they
   // were encoded for (field address, element size, C, n, outer blocks, the
   // two strides, tile width, box rows): a resize that keeps the allocation,
@@ -318,6 +325,8 @@ void allow_smem(const void* kernel, int device, size_t bytes);
 bool closed_axis(const bfvm_solver* m, int ax);
 int closed_axis_chunk(const bfvm_solver* m, int ax);
 void closed_setup(bfvm_solver* m);
+void closed_constants(const bfvm_solver* m, int a, int ch, std::vector<double>& t,
+                      std::vector<float>& tf);
 void closed_sweep(bfvm_solver* m, int ax, int fuse, int64_t z0, int64_t z1);
 // Defined in bfvm_adjoint.cu.
 void adjoint_release(bfvm_solver* m);

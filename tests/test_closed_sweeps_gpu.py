@@ -78,3 +78,19 @@ def test_a_bad_value_stays_in_its_lines():
     clean[:, 0] = clean[:, 1]
     scn.p0 = clean
     assert np.array_equal(run(scn, FP64, steps=1)[:, 1], got[:, 1])
+
+
+@pytest.mark.parametrize("shape,S", [((64, 64, 2), 1), ((50, 50, 50), 4), ((24, 24, 24), 20),
+                                     ((64, 1, 64), 3), ((9, 64, 7), 9), ((17, 5, 64), 6),
+                                     ((4, 4, 4), 300)])
+def test_grid_steps_split_planes_by_densities(shape, S):
+    """Planes of one item and of several, a last item with fewer densities,
+    more items than SMs, and constants too many to stage: several steps in
+    one launch against the oracle, agents sharing voxels included."""
+    scn = W.mixed_small(shape=shape, S=S, n_agents=300, seed=sum(shape) + S)
+    with Solver(0) as sv:
+        load_scenario(sv, scn)
+        assert sv.get_grid_steps() > 0
+        sv.step(scn.dt, 3)
+        err = O.max_rel_err(sv.get_densities(), O.oracle_run(scn, 3, 7))
+    assert np.all(err <= TOL[FP64]), err

@@ -908,8 +908,9 @@ std::string plan_key(const bfvm_batch* b, double dt, int nsteps, int flags) {
         const int v[5] = {A.ch, A.tw, A.minb, A.kind, m->chunk_nslots[a]};
         k.append(reinterpret_cast<const char*>(v), sizeof v);
       }
-      const int64_t v[8] = {m->path, m->fuse_sources, m->precision, m->n_agents,
-                            (int64_t)m->bulk_vox.size(), m->dir_unique, m->NS(), m->S};
+      const int64_t v[9] = {m->path, m->fuse_sources, m->precision, m->n_agents,
+                            (int64_t)m->bulk_vox.size(), m->dir_unique, m->NS(), m->S,
+                            m->bulk_runs};
       k.append(reinterpret_cast<const char*>(v), sizeof v);
       auto buf = [&](const DevBuf& d) {
         k.append(reinterpret_cast<const char*>(&d.ptr), sizeof d.ptr);
@@ -928,11 +929,13 @@ std::string plan_key(const bfvm_batch* b, double dt, int nsteps, int flags) {
         buf(m->chunk[a]);
         buf(m->chunk_il[a]);
         buf(m->chunk_slots[a]);
+        buf(m->closed_tab[a]);
       }
       for (const DevBuf* d : {&m->d_bulk_vox, &m->d_bulk_st, &m->d_bulk_su, &m->d_dir_vox,
                               &m->d_dir_val, &m->d_ag_vox_orig, &m->d_ag_t1, &m->d_ag_t2,
                               &m->d_ag_key, &m->d_ag_idx_in, &m->d_ag_idx, &m->d_sort_tmp,
-                              &m->d_gather, &m->d_status})
+                              &m->d_gather, &m->d_status, &m->d_bulk_vox32, &m->d_bulk_row,
+                              &m->d_bulk_tab, &m->d_bulk_runs})
         buf(*d);
       seg(m->seg_bulk);
       seg(m->seg_dir_x);

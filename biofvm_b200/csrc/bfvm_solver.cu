@@ -340,7 +340,7 @@ void build_bulk(bfvm_solver* m) {
   upload(m->d_bulk_su, m->bulk_su, st);
   // shared coefficient rows (bitwise-equal rows once): worth it when they
   // compress at least 4x and voxel indices fit int32
-  m->bulk_rows = 0;
+  m->bulk_rows = m->bulk_runs = 0;
   if (m->N() < ((int64_t)1 << 31)) {
     std::unordered_map<std::string, int> seen;
     std::vector<int> vox32(E), row(E);
@@ -374,6 +374,25 @@ void build_bulk(bfvm_solver* m) {
       upload(m->d_bulk_row, row, st);
       upload(m->d_bulk_tab, tab, st);
       m->bulk_rows = (int64_t)seen.size();
+      // runs of consecutive voxels with one row, as long as a warp takes;
+      // worth it where they fill half of one on average
+      m->bulk_runs = 0;
+      if (S <= 32) {
+        const int most = std::max(1, 32 / S * bfvm::kBulkPerLane);
+        std::vector<int> runs;
+        for (int64_t e = 0; e < E;) {
+          int64_t f = e + 1;
+          while (f < E && f - e < most && vox32[f] == vox32[f - 1] + 1 && row[f] == row[e]) ++f;
+          const int r[4] = {vox32[e], (int)(f - e), row[e], 0};
+          runs.insert(runs.end(), r, r + 4);
+          e = f;
+        }
+        const int64_t n = (int64_t)runs.size() / 4;
+        if (E * S >= 16 * n) {
+          upload(m->d_bulk_runs, runs, st);
+          m->bulk_runs = n;
+        }
+      }
     }
   }
   const int ch = m->axis[0].ch, nc = (m->nx + ch - 1) / ch;
@@ -1434,7 +1453,11 @@ void bulk_standalone(bfvm_solver* m, double dt) {
   const int64_t E = (int64_t)m->bulk_vox.size();
   if (E == 0) return;
   const int64_t work = E * m->S;
-  if (m->bulk_rows > 0)
+  if (m->bulk_runs > 0)
+    bfvm::bulk_runs_kernel<T><<<(unsigned)blocks_for(m->bulk_runs, 8), 256, 0, m->stream>>>(
+        m->p.as<T>(), m->S, 32 / m->S * m->S, (int)m->bulk_runs, m->d_bulk_runs.as<int4>(),
+        m->d_bulk_tab.as<double>(), dt);
+  else if (m->bulk_rows > 0)
     bfvm::bulk_rows_kernel<T><<<(unsigned)blocks_for(work, 256), 256, 0, m->stream>>>(
         m->p.as<T>(), m->S, E, m->d_bulk_vox32.as<int>(), m->d_bulk_row.as<int>(),
         m->d_bulk_tab.as<double>(), dt);
@@ -1451,7 +1474,7 @@ void cells_standalone(bfvm_solver* m) {
   if (A == 0) return;
   const int64_t work = A * m->S;
   bfvm::cells_kernel<T><<<(unsigned)blocks_for(work, 256), 256, 0, m->stream>>>(
-      m->p.as<T>(), m->S, A, m->d_ag_key.as<uint64_t>(), m->d_ag_idx.as<int>(),
+      m->p.as<T>(), m->S, quot_of(m->S), A, m->d_ag_key.as<uint64_t>(), m->d_ag_idx.as<int>(),
       m->d_ag_t1.as<double>(), m->d_ag_t2.as<double>());
   check_launch(m);
 }
@@ -1593,6 +1616,7 @@ int bfvm_destroy(bfvm_solver* m) {
     m->d_bulk_vox32.release();
     m->d_bulk_row.release();
     m->d_bulk_tab.release();
+    m->d_bulk_runs.release();
     m->seg_bulk.release();
     m->d_dir_vox.release();
     m->d_dir_val.release();
@@ -2246,8 +2270,8 @@ void cluster_run(bfvm_solver* m, double dt, int nsteps, int flags, int cl) {
 }
 
 constexpr int kGridMaxN = 64;  // points per axis (8-point chunks, 8 of them)
-// voxel-densities: at 64^3 x 2 = 2^19 16.1 us a step against 40 with the
-// sweep kernels, at 50^3 x 4 23.7 against 28.7
+// voxel-densities: at 64^3 x 2 = 2^19 15.9 us a step against 29.6 with the
+// sweep kernels, at 50^3 x 4 22.8 against 28.7
 constexpr int64_t kGridMaxVS = 1 << 19;
 
 constexpr size_t kGridSmemMost = 200 * 1024;

@@ -189,6 +189,10 @@ struct bfvm_solver {
   // (int32) per listed voxel, unique (S*T, U+S) rows [rows][S][2]; used by
   // the stand-alone bulk kernel when the rows compress (bulk_rows > 0)
   int64_t bulk_rows = 0;
+  // runs of consecutive listed voxels that share a row ({voxel, count, row, 0}),
+  // where they are long enough (bulk_runs > 0)
+  int64_t bulk_runs = 0;
+  bfvm_rt::DevBuf d_bulk_runs;
   bfvm_rt::DevBuf d_bulk_vox32, d_bulk_row, d_bulk_tab;
   bfvm_rt::DevSegList seg_bulk;
 

@@ -31,7 +31,7 @@ struct AdjointTape {
   int nsteps = 0, flags = 0, k = 1;
   int S = 0;
   int64_t N = 0, agents = 0, bulk = 0, nodes = 0;
-  DevBuf ckpt, tape, abar, part, acc, gt1, gt2;
+  DevBuf ckpt, tape, abar, part, acc, gt1, gt2, brow;
 };
 
 void adjoint_release(bfvm_solver* m) {
@@ -131,8 +131,24 @@ void dot_into_part(bfvm_solver* m, AdjointTape& T, const double* y, int axis) {
   const int S = m->S;
   const int threads = S * std::max(1, 256 / S);  // a multiple of S (S <= 256)
   const size_t smem = 2 * sizeof(double) * (size_t)threads;
-  adj_axis_dot_kernel<<<dot_blocks(m), threads, smem, m->stream>>>(
-      T.abar.as<double>(), y, m->nx, m->ny, m->nz, S, axis, T.part.as<double>());
+  const double* a = T.abar.as<double>();
+  if (axis == 0) {
+    adj_x_dot_kernel<<<dot_blocks(m), threads, smem, m->stream>>>(
+        a, y, m->nx, (int64_t)m->ny * m->nz, S, T.part.as<double>());
+  } else {
+    const int64_t row = (int64_t)m->nx * S, plane = row * m->ny;
+    DotAxis d{};
+    d.ls = axis == 1 ? row : plane;
+    d.os = plane;
+    d.C = (uint32_t)d.ls;
+    d.n = axis == 1 ? m->ny : m->nz;
+    d.nseg = (d.n + kDotPoints - 1) / kDotPoints;
+    d.items = (uint32_t)(d.ls * d.nseg * (axis == 1 ? m->nz : 1));
+    d.mC = quot_of(d.C);
+    d.mSeg = quot_of(d.nseg);
+    adj_axis_dot_kernel<<<dot_blocks(m), threads, smem, m->stream>>>(a, y, d, S,
+                                                                     T.part.as<double>());
+  }
   check_launch(m);
 }
 
@@ -215,6 +231,13 @@ void adjoint_backward(bfvm_solver* m, const double* seed, int seed_on_device, do
     BFVM_CUDA(cudaMemsetAsync(T.gt1.ptr, 0, (size_t)A * S * sizeof(double), st));
     BFVM_CUDA(cudaMemsetAsync(T.gt2.ptr, 0, (size_t)A * S * sizeof(double), st));
   }
+  const bool bulk = (flags & BFVM_STEP_BULK) && T.bulk > 0;
+  if (bulk && (flags & BFVM_STEP_CELLS) && A > 0) {
+    T.brow.ensure((size_t)A * sizeof(int64_t));
+    adj_bulk_rows_kernel<<<(unsigned)blocks_for(A, 256), 256, 0, st>>>(
+        A, m->d_ag_key.as<uint64_t>(), T.bulk, m->d_bulk_vox.as<int64_t>(), T.brow.as<int64_t>());
+    check_launch(m);
+  }
   const int seg_len = std::min(k, T.nsteps);
   T.tape.ensure((size_t)3 * seg_len * F);
   unsigned char* tape = T.tape.as<unsigned char>();
@@ -241,12 +264,11 @@ void adjoint_backward(bfvm_solver* m, const double* seed, int seed_on_device, do
         }
       }
       const double* in = reinterpret_cast<const double*>(j == 0 ? ck : tz(j - 1));
-      const bool bulk = (flags & BFVM_STEP_BULK) && T.bulk > 0;
       if ((flags & BFVM_STEP_CELLS) && A > 0) {
         adj_cells_kernel<<<(unsigned)blocks_for(A * S, 256), 256, 0, st>>>(
             T.abar.as<double>(), in, S, A, m->d_ag_key.as<uint64_t>(), m->d_ag_idx.as<int>(),
-            m->d_ag_t1.as<double>(), m->d_ag_t2.as<double>(), bulk ? T.bulk : 0,
-            m->d_bulk_vox.as<int64_t>(), m->d_bulk_st.as<double>(), m->d_bulk_su.as<double>(), dt,
+            m->d_ag_t1.as<double>(), m->d_ag_t2.as<double>(), bulk ? T.brow.as<int64_t>() : nullptr,
+            m->d_bulk_st.as<double>(), m->d_bulk_su.as<double>(), dt,
             T.gt1.as<double>(), T.gt2.as<double>());
         check_launch(m);
       }

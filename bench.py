@@ -338,7 +338,10 @@ def run_ours(args, world, rank, local):
     # warm-up (also builds the Thomas coefficients and the device lists), then
     # the per-axis kernel choice timed on this field (which is restored)
     sv.step(dt, args.warmup, STEP_ALL)
+    untuned = [(sv.get_sweep_kernel(ax),) + tuple(sv.get_sweep_config(ax)) for ax in range(3)]
     tuned = sv.tune_sweeps(dt, 3) if not args.no_tune else [(0, 0, 0, 0, 0)] * 3
+    # an axis that the tuner left as it was runs the default, closed-form kernel
+    tuned = [(0,) + tuple(t[1:]) if tuple(t) == u else t for t, u in zip(tuned, untuned)]
     if args.sweep_chunks:
         # only where the chunk length changes: a set configuration also
         # returns the axis to its default kernel kind
@@ -1106,7 +1109,10 @@ def run_lod2d(args, world, rank, local):
         sv.simulate_diffusion_decay_2d(dt)
     # the sweep kernels timed on this plane (after the first step fixed the
     # LOD_2D Thomas coefficients; the field is restored)
+    untuned = [(sv.get_sweep_kernel(ax),) + tuple(sv.get_sweep_config(ax)) for ax in range(3)]
     tuned = sv.tune_sweeps(dt, 3) if not args.no_tune else []
+    # an axis that the tuner left as it was runs the default, closed-form kernel
+    tuned = [(0,) + tuple(t[1:]) if tuple(t) == u else t for t, u in zip(tuned, untuned)]
     sv.set_slab_planes(0)
     sv.synchronize()
     e0 = torch.cuda.Event(enable_timing=True)

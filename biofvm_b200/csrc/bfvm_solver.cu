@@ -39,7 +39,8 @@ std::vector<int> segment_offsets(int64_t nlines, int nchunks, int ch,
   return off;
 }
 
-// Chunk length CH (points per thread) and block width TW (columns per block)
+// Shapes of the tabulated kernels, for the axes closed_sweep does not take:
+// chunk length CH (points per thread) and block width TW (columns per block)
 // per axis; a block is TW x NC threads with NC = ceil(n/CH) <= 512/TW.  The y
 // and z sweeps of long lines take CH = 32 (fewer chunks to join per line).
 // x takes the row kernel with CH = 32 where it was measured faster than the
@@ -2896,7 +2897,7 @@ int bfvm_get_row_build(bfvm_solver* m, int* requested, int* effective) {
     require(requested != nullptr && effective != nullptr, "bad arguments");
     *requested = m->axis[0].build;
     const RowsPlan P = plan_rows(m);
-    *effective = P.ok ? P.build : 0;
+    *effective = P.ok && !closed_axis(m, 0) ? P.build : 0;
   });
 }
 

@@ -237,7 +237,7 @@ class Solver:
 
     def get_sweep_kernel(self, axis: int) -> int:
         """The kernel `axis` sweeps with under PATH_AUTO: 0 for the default
-        (the register kernel), else a PATH_* value."""
+        (the closed-form kernels), else a PATH_* value."""
         k = ctypes.c_int()
         call("bfvm_get_sweep_kernel", self._h, axis, ctypes.byref(k))
         return k.value

@@ -287,8 +287,8 @@ BFVM_API int bfvm_get_stream(bfvm_solver* m, void** stream);
 BFVM_API int bfvm_get_launch_count(bfvm_solver* m, int64_t* count);
 
 /* Sweep tuner (no counterpart in the reference): for each axis, times every
- * kernel that can run it -- the register kernel at each chunk length and
- * block width, the TMA-fed kernel and the direct kernel at each chunk
+ * kernel that can run it -- the closed-form default, the register kernel at
+ * each chunk length and block width, the TMA-fed kernel and the direct kernel at each chunk
  * length -- over reps sweeps of this solver's own field, and keeps the
  * fastest for later steps (used while the kernel path is BFVM_PATH_AUTO);
  * then the slab thickness of bfvm_set_slab_planes and bfvm_set_fuse_sources,
@@ -335,14 +335,11 @@ BFVM_API int bfvm_get_cluster_steps(bfvm_solver* m, int* blocks);
 /* Whole steps of a small field in one cooperative launch over all SMs: under
  * BFVM_PATH_AUTO, bfvm_step runs all its steps in one launch when the FP64
  * field has at most 2^19 voxel-densities and no axis has more than 64
- * points (and the cluster mode above is not in use).  Each step is a phase of
- * bulk and cell updates, then one phase per axis in which blocks solve tiles
- * of lines in 4- or 8-point chunks as the sweep kernels do (Dirichlet values applied
- * as the chunks load), separated by grid-wide barriers; after the first
- * step the bulk and cell updates are applied as the previous z phase stores
- * its points.  On by default (17.7 vs 24.7 us per step at 50^3 x 1 on a
- * B200 with 1000 agents, faster than the sweep
- * kernels up to 2^19 voxel-densities); enable = 0 gives back the sweep
+ * points (and the cluster mode above is not in use).  Each step is two phases
+ * separated by grid-wide barriers: xy planes in shared memory (bulk and cell
+ * updates and Dirichlet values as they load, then the x and y lines), and
+ * tiles of z columns.  On by default (15.9 vs 29.6 us per step at 64^3 x 2 on
+ * a B200, 22.8 vs 28.7 at 50^3 x 4); enable = 0 gives back the sweep
  * kernels.  bfvm_get_grid_steps gives the launch's block count for this
  * solver now (0: not used). */
 BFVM_API int bfvm_set_grid_steps(bfvm_solver* m, int enable);

@@ -94,3 +94,22 @@ def test_grid_steps_split_planes_by_densities(shape, S):
         sv.step(scn.dt, 3)
         err = O.max_rel_err(sv.get_densities(), O.oracle_run(scn, 3, 7))
     assert np.all(err <= TOL[FP64]), err
+
+
+def test_many_row_tiles_a_place():
+    """x rows enough for several blocks a place on the device (32,768 tiles)
+    against the same step in slabs of 16 planes (2,048 tiles each, one block a
+    place): the same tiles, the same bits."""
+    rng = np.random.default_rng(11)
+    shape, S = (96, 256, 256), 16
+    scn = W.mixed_small(shape=shape, S=S, n_agents=0, seed=12, bulk=False, dirichlet=False)
+    p = rng.uniform(0.5, 1.5, (int(np.prod(shape)), S))
+    got = []
+    for planes in (0, 16):
+        with Solver(0) as sv:
+            load_scenario(sv, scn)
+            sv.set_densities(p)
+            sv.set_slab_planes(planes)
+            sv.step(scn.dt, 1)
+            got.append(sv.get_densities())
+    assert np.array_equal(got[0], got[1])

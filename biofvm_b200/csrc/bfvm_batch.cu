@@ -904,13 +904,19 @@ std::string plan_key(const bfvm_batch* b, double dt, int nsteps, int flags) {
   if (b->cfg.mode == BFVM_BATCH_BRANCHES || persistent_mode(b->cfg.mode))
     for (const bfvm_solver* m : b->inst) {
       for (int a = 0; a < 3; ++a) {
+        // the kernel that sweeps the axis (the closed-form one at its chunk
+        // length, or the axis's own choice) and the chunk length the
+        // Dirichlet segments it reads are laid out for
         const Axis& A = m->axis[a];
-        const int v[5] = {A.ch, A.tw, A.minb, A.kind, m->chunk_nslots[a]};
+        const int v[9] = {A.ch,     A.tw,    A.minb,
+                          A.kind,   m->chunk_nslots[a],
+                          A.stages, A.build, closed_axis(m, a) ? closed_axis_chunk(m, a) : 0,
+                          a < 2 ? m->dir_ch[a] : 0};
         k.append(reinterpret_cast<const char*>(v), sizeof v);
       }
-      const int64_t v[9] = {m->path, m->fuse_sources, m->precision, m->n_agents,
-                            (int64_t)m->bulk_vox.size(), m->dir_unique, m->NS(), m->S,
-                            m->bulk_runs};
+      const int64_t v[13] = {m->path, m->fuse_sources, m->precision, m->n_agents,
+                             (int64_t)m->bulk_vox.size(), m->dir_unique, m->nx, m->ny, m->nz,
+                             m->S, m->bulk_runs, m->slab_planes, m->zs_ranks};
       k.append(reinterpret_cast<const char*>(v), sizeof v);
       auto buf = [&](const DevBuf& d) {
         k.append(reinterpret_cast<const char*>(&d.ptr), sizeof d.ptr);

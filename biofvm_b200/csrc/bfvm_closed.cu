@@ -36,10 +36,11 @@ int closed_chunk(const bfvm_solver* m, int a) {
 }  // namespace
 
 // Whether the closed-form kernels sweep this axis: the default choice
-// (BFVM_PATH_AUTO, no configuration set on the axis), lines the chunked
-// kernels take, whole lines (a z slab's carries come from the other slabs).
+// (BFVM_PATH_AUTO, no configuration set on the axis), coefficients that have
+// the closed form (closed_coefficients), lines the chunked kernels take, whole
+// lines (a z slab's carries come from the other slabs).
 bool closed_axis(const bfvm_solver* m, int ax) {
-  if (m->path != BFVM_PATH_AUTO || m->axis[ax].user) return false;
+  if (m->path != BFVM_PATH_AUTO || m->axis[ax].user || !m->closed_ok) return false;
   if (ax == 2 && m->zs_ranks > 0) return false;
   if (ax == 0 && m->fuse_sources) return false;
   const int n = axis_points(m, ax);
@@ -48,10 +49,45 @@ bool closed_axis(const bfvm_solver* m, int ax) {
 
 int closed_axis_chunk(const bfvm_solver* m, int ax) { return closed_chunk(m, ax); }
 
+namespace {
+
+// c1 = dt D / dx^2 and c2 = dt decay / 3 (/ 2 for LOD_2D) of density s as the
+// Thomas setup has them (BioFVM_solvers.cpp:105-126; dx on every axis), and
+// the slope r = c1 / d, d the larger root of d^2 - (1 + 2 c1 + c2) d + c1^2,
+// rounded to the arithmetic type.
+struct Slope {
+  long double c1, c2, r;
+};
+Slope closed_slope(const bfvm_solver* m, int s) {
+  Slope k;
+  k.c1 = (long double)m->h_c1[0][s];
+  k.c2 = (long double)m->setup_decay[s] * m->setup_dt / (m->setup_dims == 2 ? 2 : 3);
+  const long double b = 1 + 2 * k.c1 + k.c2;
+  const long double d = (b + std::sqrt((1 + k.c2) * (1 + k.c2 + 4 * k.c1))) / 2;
+  const long double r = k.c1 / d;
+  k.r = m->math_elem() == 4 ? (long double)(float)r : (long double)(double)r;
+  return k;
+}
+
+// Whether every density of the setup has the closed form: c1 >= 0 and
+// 1 + c2 > 0, which give a real slope in [0, 1), and a slope that is still
+// below 1 when rounded (FP32: c1 up to about 1e15).  Others (a negative
+// diffusion coefficient, a negative decay rate of 3 / dt or more) are solved
+// by elimination, which has a result wherever its divisors are not zero.
+// Written so that a NaN answers false.
+bool closed_coefficients(const bfvm_solver* m) {
+  for (int s = 0; s < m->S; ++s) {
+    const Slope k = closed_slope(m, s);
+    if (!(k.c1 >= 0 && 1 + k.c2 > 0 && k.r >= 0 && k.r < 1)) return false;
+  }
+  return true;
+}
+
+}  // namespace
+
 // Constants of axis a for ch-point chunks (ClosedCoef: cst, then pw) from the
-// coefficients of the Thomas setup (BioFVM_solvers.cpp:105-126: c1 = dt D /
-// dx^2, c2 = dt decay / 3, or / 2 for LOD_2D), in extended precision and
-// rounded once: to t, in FP32 to the pairs tf.
+// slopes of the Thomas setup, in extended precision and rounded once: to t, in
+// FP32 to the pairs tf.
 void closed_constants(const bfvm_solver* m, int a, int ch, std::vector<double>& t,
                       std::vector<float>& tf) {
   const int S = m->S, n = axis_points(m, a), nc = (n + ch - 1) / ch;
@@ -60,13 +96,8 @@ void closed_constants(const bfvm_solver* m, int a, int ch, std::vector<double>& 
   t.assign(count, 0.0);
   tf.assign(fp32 ? 2 * count : 0, 0.0f);
   for (int s = 0; s < S; ++s) {
-    const long double c1 = (long double)m->h_c1[a][s];
-    const long double c2 =
-        (long double)m->setup_decay[s] * m->setup_dt / (m->setup_dims == 2 ? 2 : 3);
-    // r = c1 / d with d the larger root of d^2 - (1 + 2 c1 + c2) d + c1^2
-    const long double b = 1 + 2 * c1 + c2;
-    const long double d = (b + std::sqrt((1 + c2) * (1 + c2 + 4 * c1))) / 2;
-    const long double r = fp32 ? (long double)(float)(c1 / d) : (long double)(double)(c1 / d);
+    const Slope slope = closed_slope(m, s);
+    const long double r = slope.r, c2 = slope.c2;
     auto put = [&](size_t i, long double x) {
       t[i] = (double)x;
       if (fp32) {
@@ -90,6 +121,8 @@ void closed_constants(const bfvm_solver* m, int a, int ch, std::vector<double>& 
 void closed_setup(bfvm_solver* m) {
   std::vector<double> t;
   std::vector<float> tf;
+  m->closed_ok = closed_coefficients(m);
+  if (!m->closed_ok) return;
   for (int a = 0; a < 3; ++a) {
     if (axis_points(m, a) > 1024) continue;
     closed_constants(m, a, closed_chunk(m, a), t, tf);

@@ -2294,7 +2294,8 @@ struct GridPlan {
 GridPlan plan_grid(bfvm_solver* m) {
   GridPlan P;
   if (!m->grid_steps || m->path != BFVM_PATH_AUTO || m->precision != BFVM_FP64 ||
-      m->lod_dims != 3 || !m->uniform || m->fuse_sources || m->slab_planes > 0 || m->zs_ranks > 0)
+      m->lod_dims != 3 || !m->uniform || m->fuse_sources || m->slab_planes > 0 ||
+      m->zs_ranks > 0 || !m->closed_ok)
     return P;
   if (m->nx > kGridMaxN || m->ny > kGridMaxN || m->nz > kGridMaxN) return P;
   if ((int64_t)m->NS() > kGridMaxVS || cluster_blocks(m) > 0) return P;
@@ -2482,10 +2483,13 @@ int bfvm_step(bfvm_solver* m, double dt, int nsteps, int flags) {
       cluster_run(m, dt, nsteps, flags, cl);
       return;
     }
+    if (nsteps > 0 && !m->setup_done) {  // the setup says whether the grid steps apply
+      check_lod_mesh(m);
+      thomas_setup(m, dt);
+    }
     const GridPlan grid = nsteps > 0 ? plan_grid(m) : GridPlan();
     if (grid.blocks > 0) {
       check_lod_mesh(m);
-      if (!m->setup_done) thomas_setup(m, dt);
       build_all(m);
       grid_run(m, dt, nsteps, flags, grid);
       return;

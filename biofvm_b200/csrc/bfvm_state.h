@@ -176,8 +176,10 @@ struct bfvm_solver {
   int chunk_nslots[3] = {0, 0, 0};
   bfvm_rt::Axis axis[3];
   // constants of the closed-form sweeps per axis (cst [S][8], pw [chunks][S][2]),
-  // built with the Thomas setup; lod_dims at that setup
+  // built with the Thomas setup; whether its coefficients have the closed
+  // form; lod_dims at that setup
   bfvm_rt::DevBuf closed_tab[3];
+  bool closed_ok = true;
   int setup_dims = 3;
 
   // bulk sources/sinks: non-identity voxels, ascending

@@ -132,21 +132,33 @@ class ClockSampler:
 TRAFFIC_PROFILE = os.path.join(ROOT, "profiles", "sweeps_traffic_lod256.json")
 
 
-def ncu_traffic(axis_key: str, kernel_kind: int, chunk: int, row_build: int):
+def swept_by(sv, axis: int) -> dict:
+    """The kernel that sweeps an axis now: "default" for the closed-form one,
+    else the tabulated kernel the tuner or a set configuration chose."""
+    closed = sv.get_closed_sweep(axis)
+    chunk, columns, min_blocks, stages = sv.get_sweep_config(axis)
+    if closed:
+        return {"axis": "xyz"[axis], "kernel": "default", "chunk": closed}
+    return {"axis": "xyz"[axis],
+            "kernel": ["tabulated", "register", "tma", "direct"][sv.get_sweep_kernel(axis)],
+            "chunk": chunk, "columns": columns, "min_blocks": min_blocks, "row_stages": stages}
+
+
+def ncu_traffic(axis_key: str, kernel: str, chunk: int, row_build: int):
     """DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch
     of the sweep kernel of an axis at the full 256^3 x 10 size, from the
     one-pass ncu capture recorded in profiles/sweeps_traffic_lod256.json
     (the capture's command is in the file).  None when the file lacks the
     axis or the capture ran another kernel than the one timed here: another
-    kernel kind (kernel_kind: the tuner's choice, a BFVM_PATH_* value, 0 =
-    the default, which the capture ran), chunk length or x row-kernel
-    build."""
+    kind (as swept_by names it; the capture's path 0 is "default"), chunk
+    length or x row-kernel build."""
     if not os.path.exists(TRAFFIC_PROFILE):
         return None, None
     with open(TRAFFIC_PROFILE) as f:
         d = json.load(f)
     k = d.get("launches", {}).get(axis_key)
-    if not k or (kernel_kind != 0 and kernel_kind != k.get("path")):
+    kinds = ["default", "register", "tma", "direct"]
+    if not k or kernel not in kinds or kinds.index(kernel) != k.get("path"):
         return None, None
     if k.get("chunk") != chunk or (axis_key == "x_sweep" and k.get("row_build") != row_build):
         return None, None
@@ -338,19 +350,18 @@ def run_ours(args, world, rank, local):
     # warm-up (also builds the Thomas coefficients and the device lists), then
     # the per-axis kernel choice timed on this field (which is restored)
     sv.step(dt, args.warmup, STEP_ALL)
-    untuned = [(sv.get_sweep_kernel(ax),) + tuple(sv.get_sweep_config(ax)) for ax in range(3)]
-    tuned = sv.tune_sweeps(dt, 3) if not args.no_tune else [(0, 0, 0, 0, 0)] * 3
-    # an axis that the tuner left as it was runs the default, closed-form kernel
-    tuned = [(0,) + tuple(t[1:]) if tuple(t) == u else t for t, u in zip(tuned, untuned)]
+    if not args.no_tune:
+        sv.tune_sweeps(dt, 3)
     if args.sweep_chunks:
         # only where the chunk length changes: a set configuration also
-        # returns the axis to its default kernel kind
+        # takes the axis off its default kernel
         for ax, ch in enumerate(int(c) for c in args.sweep_chunks.split(",")):
-            if sv.get_sweep_config(ax)[0] != ch:
+            if swept_by(sv, ax)["chunk"] != ch:
                 sv.set_sweep_config(ax, ch, 16, 1)
     if args.row_build is not None:
         sv.set_row_build(args.row_build)
     row_build = sv.get_row_build()
+    tuned = [swept_by(sv, ax) for ax in range(3)]
     sv.synchronize()
 
     launches0 = sv.launch_count
@@ -386,8 +397,8 @@ def run_ours(args, world, rank, local):
     hbm, peak_kind = peaks()
     achieved = sweeps_in[dom] * BYTES_PER_VS_SWEEP * N * S / (per[dom] / 1e3) / 1e9
     dom_axis = {"x_sweep": 0, "y_sweep": 1, "z_sweep": 2}.get(dom)
-    traffic, traffic_kernel = (ncu_traffic(dom, tuned[dom_axis][0],
-                                           sv.get_sweep_config(dom_axis)[0], row_build[1])
+    traffic, traffic_kernel = (ncu_traffic(dom, tuned[dom_axis]["kernel"],
+                                           tuned[dom_axis]["chunk"], row_build[1])
                                if dom_axis is not None else (None, None))
 
     # end to end through the C ABI with host buffers: every step uploads the
@@ -475,9 +486,7 @@ def run_ours(args, world, rank, local):
                                            "launch at 256^3 x 10)" if traffic else None,
                          "algorithmic_bytes_per_launch": sweeps_in[dom] * BYTES_PER_VS_SWEEP * N * S},
             "kernel_ms": per,
-            "tuned_sweeps": [{"axis": "xyz"[i], "kernel": ["default", "register", "tma", "direct"][k],
-                              "chunk": ch, "columns": tw, "min_blocks": mb, "row_stages": st}
-                             for i, (k, ch, tw, mb, st) in enumerate(tuned)],
+            "tuned_sweeps": tuned,
             "row_build": dict(zip(("requested", "effective"), row_build)),
             "slab_planes": sv.get_slab_planes(), "fuse_sources": sv.get_fuse_sources(),
             "gpu_launches": int(launches),
@@ -1109,10 +1118,9 @@ def run_lod2d(args, world, rank, local):
         sv.simulate_diffusion_decay_2d(dt)
     # the sweep kernels timed on this plane (after the first step fixed the
     # LOD_2D Thomas coefficients; the field is restored)
-    untuned = [(sv.get_sweep_kernel(ax),) + tuple(sv.get_sweep_config(ax)) for ax in range(3)]
-    tuned = sv.tune_sweeps(dt, 3) if not args.no_tune else []
-    # an axis that the tuner left as it was runs the default, closed-form kernel
-    tuned = [(0,) + tuple(t[1:]) if tuple(t) == u else t for t, u in zip(tuned, untuned)]
+    if not args.no_tune:
+        sv.tune_sweeps(dt, 3)
+    tuned = [swept_by(sv, ax) for ax in range(2)]
     sv.set_slab_planes(0)
     sv.synchronize()
     e0 = torch.cuda.Event(enable_timing=True)
@@ -1139,10 +1147,7 @@ def run_lod2d(args, world, rank, local):
             "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded)",
             "config": {"workload": f"lod2d: {n}^2 voxels x {S} substrates FP64",
                        "l2": "field larger than L2; no flush"},
-            "tuned_sweeps": [{"axis": "xy"[i], "kernel": ["default", "register", "tma",
-                                                          "direct"][k],
-                              "chunk": ch, "columns": tw} for i, (k, ch, tw, *_) in
-                             enumerate(tuned[:2])],
+            "tuned_sweeps": tuned,
             "roofline": {"bound": "hbm", "kernel": "x and y sweeps of the plane",
                          "achieved": achieved, "peak": hbm, "peak_kind": peak_kind,
                          "unit": "GB/s", "frac": achieved / hbm, "traffic": None},

@@ -105,6 +105,7 @@ SIGNATURES = {
     "bfvm_get_grid_steps": (c_int, [_P, _IP]),
     "bfvm_profile_step": (c_int, [_P, c_double, c_int, c_int, _DP]),
     "bfvm_tune_sweeps": (c_int, [_P, c_double, c_int]),
+    "bfvm_get_closed_sweep": (c_int, [_P, c_int, _IP]),
     "bfvm_get_sweep_kernel": (c_int, [_P, c_int, _IP]),
     "bfvm_compute_all_gradient_vectors": (c_int, [_P]),
     "bfvm_get_gradient_vectors": (c_int, [_P, _DP]),

@@ -2872,6 +2872,13 @@ int bfvm_tune_sweeps(bfvm_solver* m, double dt, int reps) {
   return SOLVER_CALL(m, tune_sweeps(m, dt, reps));
 }
 
+int bfvm_get_closed_sweep(bfvm_solver* m, int axis, int* chunk) {
+  return SOLVER_CALL(m, {
+    require(axis >= 0 && axis < 3 && chunk != nullptr, "bad arguments");
+    *chunk = m->N() > 0 && closed_axis(m, axis) ? closed_axis_chunk(m, axis) : 0;
+  });
+}
+
 int bfvm_get_sweep_kernel(bfvm_solver* m, int axis, int* kind) {
   return SOLVER_CALL(m, {
     require(axis >= 0 && axis < 3 && kind != nullptr, "bad arguments");

@@ -224,7 +224,8 @@ class Solver:
     def tune_sweeps(self, dt: float, reps: int = 5):
         """Picks each axis's fastest sweep kernel by timing them on this field
         (which is restored); returns [(kernel, chunk, columns, min_blocks,
-        row-kernel ring stages)] per axis."""
+        row-kernel ring stages)] per axis, the tabulated kernels' choice (not
+        in use where `get_closed_sweep` is not 0)."""
         call("bfvm_tune_sweeps", self._h, dt, reps)
         out = []
         for ax in range(3):
@@ -235,9 +236,17 @@ class Solver:
             out.append((k.value, cfg[0], cfg[1], cfg[2], cfg[3]))
         return out
 
+    def get_closed_sweep(self, axis: int) -> int:
+        """Points per thread of the closed-form kernel that sweeps `axis` now,
+        0 where a tabulated kernel does (`get_sweep_kernel`)."""
+        chunk = ctypes.c_int()
+        call("bfvm_get_closed_sweep", self._h, axis, ctypes.byref(chunk))
+        return chunk.value
+
     def get_sweep_kernel(self, axis: int) -> int:
-        """The kernel `axis` sweeps with under PATH_AUTO: 0 for the default
-        (the closed-form kernels), else a PATH_* value."""
+        """The tabulated kernel of `axis` under PATH_AUTO, which runs where
+        `get_closed_sweep` is 0: 0 by axis (register kernel for x, TMA-fed for
+        y and z), else a PATH_* value."""
         k = ctypes.c_int()
         call("bfvm_get_sweep_kernel", self._h, axis, ctypes.byref(k))
         return k.value

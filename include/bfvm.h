@@ -294,9 +294,18 @@ BFVM_API int bfvm_get_launch_count(bfvm_solver* m, int64_t* count);
  * then the slab thickness of bfvm_set_slab_planes and bfvm_set_fuse_sources,
  * over whole steps.
  * The field is saved before and restored after; bfvm_set_sweep_config or
- * a resize resets the choice.  bfvm_get_sweep_kernel returns the axis's
- * kernel (0 = the default choice, else a BFVM_PATH_* value). */
+ * a resize resets the choice. */
 BFVM_API int bfvm_tune_sweeps(bfvm_solver* m, double dt, int reps);
+/* What sweeps an axis now.  bfvm_get_closed_sweep: points per thread of the
+ * closed-form kernel, or 0 where one of the tabulated kernels runs (a kernel
+ * path other than AUTO, a choice of the tuner or of bfvm_set_sweep_config,
+ * sources fused into x, a z slab's z, more than 1024 points, coefficients of
+ * the last setup without the closed form).  bfvm_get_sweep_kernel and
+ * bfvm_get_sweep_config then say which: the axis's tabulated kernel under
+ * BFVM_PATH_AUTO (0 = by axis: register kernel for x, TMA-fed for y and z,
+ * else a BFVM_PATH_* value) and its launch shape.  While the closed-form
+ * kernel runs they hold the choice that would take its place. */
+BFVM_API int bfvm_get_closed_sweep(bfvm_solver* m, int axis, int* chunk);
 BFVM_API int bfvm_get_sweep_kernel(bfvm_solver* m, int axis, int* kind);
 
 /* Runs the x and y sweeps of a step slab by slab: for each slab of `planes`

@@ -1,0 +1,82 @@
+"""Which kernel sweeps an axis, and that a change of it keeps the results:
+the closed form by default, the tabulated kernels where a path, a
+configuration, fused sources or a length past 1024 points asks for them, and
+the chunk length following added densities after a first step.  Steps against
+the oracle at the suite's 1e-12."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from biofvm_b200 import Solver, load_scenario
+from biofvm_b200 import workloads as W
+from biofvm_b200._abi import PATH_AUTO, PATH_TMA
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def swept(sv):
+    return [sv.get_closed_sweep(ax) for ax in range(3)]
+
+
+def check_step(sv, scn):
+    step = dataclasses.replace(scn, p0=sv.get_densities())
+    sv.step(scn.dt, 1)
+    err = O.max_rel_err(sv.get_densities(), O.oracle_run(step, 1, 7))
+    assert np.all(err <= 1e-12), err
+
+
+@pytest.mark.parametrize("shape,S", [((96, 20, 12), 4), ((160, 12, 10), 5), ((64, 20, 12), 6)])
+def test_what_sweeps_an_axis(shape, S):
+    scn = W.mixed_small(shape=shape, S=S, n_agents=200, seed=sum(shape) + S)
+    with Solver(0) as sv:
+        load_scenario(sv, scn)
+        sv.set_grid_steps(False)
+        assert swept(sv) == [16, 16, 16]
+        check_step(sv, scn)
+        for path, expect in ((PATH_TMA, [0, 0, 0]), (PATH_AUTO, [16, 16, 16])):
+            sv.set_kernel_path(path)
+            assert swept(sv) == expect
+            check_step(sv, scn)
+        sv.set_fuse_sources(True)
+        assert swept(sv) == [0, 16, 16]
+        check_step(sv, scn)
+        sv.set_fuse_sources(False)
+        sv.set_sweep_config(1, 8, 16)
+        assert swept(sv) == [16, 0, 16]
+        check_step(sv, scn)
+
+
+def test_long_lines_and_coefficients():
+    scn = W.mixed_small(shape=(1100, 5, 4), S=2, n_agents=50, seed=4)
+    with Solver(0) as sv:
+        load_scenario(sv, scn)
+        assert swept(sv) == [0, 16, 16]
+        check_step(sv, scn)
+        sv.set_coefficients(np.array([1.0, -1.0]), np.zeros(2))
+        sv.reset_diffusion_setup()
+        sv.step(scn.dt, 1)
+        assert swept(sv) == [0, 0, 0]
+
+
+def test_chunks_follow_an_added_density():
+    """x of 64 points takes 16-point chunks while 32-point ones would leave
+    fewer than 128 threads an SM (15,360 in all with one density, 30,720 with
+    two), 32-point chunks from the second density on."""
+    scn = W.mixed_small(shape=(64, 96, 80), S=2, n_agents=0, seed=8, bulk=False, dirichlet=False)
+    m = scn.mesh
+    with Solver(0) as sv:
+        sv.resize_densities(1)
+        sv.resize_space(m.x0, m.x1, m.y0, m.y1, m.z0, m.z1, m.dx, m.dy, m.dz)
+        sv.set_coefficients(scn.D[:1], scn.decay[:1])
+        sv.set_densities(scn.p0[:, :1])
+        sv.set_grid_steps(False)
+        first = sv.get_closed_sweep(0)
+        sv.step(scn.dt, 1)
+        sv.add_density(float(scn.D[1]), float(scn.decay[1]))
+        assert (first, sv.get_closed_sweep(0)) == (16, 32)
+        p = sv.get_densities()
+        p[:, 1] = scn.p0[:, 1]
+        sv.set_densities(p)
+        check_step(sv, scn)

@@ -86,6 +86,7 @@ SIGNATURES = {
     "bfvm_reset_diffusion_setup": (c_int, [_P]),
     "bfvm_set_precision": (c_int, [_P, c_int]),
     "bfvm_set_sweep_config": (c_int, [_P, c_int, c_int, c_int, c_int]),
+    "bfvm_reset_sweep_config": (c_int, [_P, c_int]),
     "bfvm_get_sweep_config": (c_int, [_P, c_int, _IP]),
     "bfvm_set_row_stages": (c_int, [_P, c_int]),
     "bfvm_set_row_build": (c_int, [_P, c_int]),

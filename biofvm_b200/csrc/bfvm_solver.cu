@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdlib>
 #include <cstdio>
@@ -2704,6 +2705,19 @@ int bfvm_set_sweep_config(bfvm_solver* m, int axis, int chunk, int columns, int 
     A.kind = 0;
     A.stages = 0;
     A.user = true;
+  });
+}
+
+int bfvm_reset_sweep_config(bfvm_solver* m, int axis) {
+  return SOLVER_CALL(m, {
+    require(axis >= 0 && axis < 3, "axis must be 0, 1 or 2");
+    const std::array<Axis, 3> set = {m->axis[0], m->axis[1], m->axis[2]};
+    m->axis[axis].user = false;
+    m->axis[axis].minb = 1;
+    choose_axes(m);
+    for (int a = 0; a < 3; ++a)
+      if (a != axis) m->axis[a] = set[a];
+    m->bulk_dirty = m->dir_dirty = m->ag_seg_dirty = true;
   });
 }
 

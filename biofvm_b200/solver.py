@@ -254,6 +254,11 @@ class Solver:
     def set_sweep_config(self, axis: int, chunk: int, columns: int, min_blocks: int = 1) -> None:
         call("bfvm_set_sweep_config", self._h, axis, chunk, columns, min_blocks)
 
+    def reset_sweep_config(self, axis: int) -> None:
+        """Gives `axis` back to the default sweep after `set_sweep_config` or
+        the tuner."""
+        call("bfvm_reset_sweep_config", self._h, axis)
+
     def get_sweep_config(self, axis: int):
         """(chunk, columns, min_blocks, row-kernel ring stages) of `axis`."""
         cfg = (ctypes.c_int * 4)()

@@ -236,9 +236,12 @@ BFVM_API int bfvm_set_precision(bfvm_solver* m, int precision);
  * whose OpenMP loops have no tunables): chunk = points per thread (8, 16,
  * 32), columns = lines per block (8..64), min_blocks = resident blocks per SM
  * the kernel is compiled for (1, 2).  Kept until the next resize.  The
- * default is chosen from the axis length; the autotuner sets this. */
+ * default is chosen from the axis length; the autotuner sets this.  The axis
+ * then runs a tabulated kernel of that shape until bfvm_reset_sweep_config
+ * gives it back to the default. */
 BFVM_API int bfvm_set_sweep_config(bfvm_solver* m, int axis, int chunk, int columns,
                                    int min_blocks);
+BFVM_API int bfvm_reset_sweep_config(bfvm_solver* m, int axis);
 /* config[4] = chunk, columns, min_blocks, and the tiles in the x row
  * kernel's shared-memory ring (2, or 3 where the tuner found it faster) */
 /* Tiles in the x row kernel's shared-memory ring: 2 (default) or 3 (one more
@@ -293,8 +296,8 @@ BFVM_API int bfvm_get_launch_count(bfvm_solver* m, int64_t* count);
  * fastest for later steps (used while the kernel path is BFVM_PATH_AUTO);
  * then the slab thickness of bfvm_set_slab_planes and bfvm_set_fuse_sources,
  * over whole steps.
- * The field is saved before and restored after; bfvm_set_sweep_config or
- * a resize resets the choice. */
+ * The field is saved before and restored after; bfvm_set_sweep_config,
+ * bfvm_reset_sweep_config or a resize resets the choice. */
 BFVM_API int bfvm_tune_sweeps(bfvm_solver* m, double dt, int reps);
 /* What sweeps an axis now.  bfvm_get_closed_sweep: points per thread of the
  * closed-form kernel, or 0 where one of the tabulated kernels runs (a kernel

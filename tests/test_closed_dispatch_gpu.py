@@ -80,3 +80,34 @@ def test_chunks_follow_an_added_density():
         p[:, 1] = scn.p0[:, 1]
         sv.set_densities(p)
         check_step(sv, scn)
+
+
+def test_an_axis_goes_back_to_the_default():
+    """After a set configuration and after the tuner, with the fields of a
+    solver that never left the default."""
+    scn = W.mixed_small(shape=(40, 36, 130), S=2, n_agents=100, seed=21)
+    with Solver(0) as sv, Solver(0) as plain:
+        for s in (sv, plain):
+            load_scenario(s, scn)
+            s.set_grid_steps(False)
+        shapes = [sv.get_sweep_config(ax) for ax in range(3)]
+        for ax in range(3):
+            sv.set_sweep_config(ax, 16, 16, 2)
+        assert swept(sv) == [0, 0, 0]
+        for ax in range(3):
+            sv.reset_sweep_config(ax)
+        assert swept(sv) == swept(plain) == [16, 16, 16]
+        assert [sv.get_sweep_config(ax) for ax in range(3)] == shapes
+        sv.step(scn.dt, 2)
+        sv.tune_sweeps(scn.dt, 1)
+        sv.set_fuse_sources(False)
+        for ax in range(3):
+            sv.reset_sweep_config(ax)
+        sv.set_slab_planes(0)
+        assert swept(sv) == [16, 16, 16]
+        sv.step(scn.dt, 1)
+        plain.step(scn.dt, 3)
+        got = sv.get_densities()
+        assert np.array_equal(got, plain.get_densities())
+    err = O.max_rel_err(got, O.oracle_run(scn, 3, 7))
+    assert np.all(err <= 1e-12), err

@@ -2740,6 +2740,7 @@ void tune_sweeps(bfvm_solver* m, double dt, int reps) {
   const int saved_slab = m->slab_planes;
   const int saved_fuse = m->fuse_sources;
   m->path = BFVM_PATH_AUTO;
+  m->fuse_sources = 0;  // x is timed as the default sweeps it; fusion is settled last
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   BFVM_CUDA(cudaEventCreate(&e0));
   BFVM_CUDA(cudaEventCreate(&e1));
@@ -2856,6 +2857,8 @@ void tune_sweeps(bfvm_solver* m, double dt, int reps) {
         }
       }
       m->fuse_sources = best_f;
+    } else {
+      m->fuse_sources = saved_fuse;
     }
   } catch (...) {
     m->fuse_sources = saved_fuse;

@@ -111,3 +111,17 @@ def test_an_axis_goes_back_to_the_default():
         assert np.array_equal(got, plain.get_densities())
     err = O.max_rel_err(got, O.oracle_run(scn, 3, 7))
     assert np.all(err <= 1e-12), err
+
+
+def test_the_tuner_times_the_default_x_sweep_with_fusion_set():
+    """x of this field takes 31 us in closed form and 49 us in the best of the
+    tabulated kernels: the tuner must find it also where sources were set to be
+    fused into x (there is nothing to fuse, so that setting stays)."""
+    scn = W.mixed_small(shape=(161, 97, 123), S=3, n_agents=0, seed=9, bulk=False)
+    with Solver(0) as sv:
+        load_scenario(sv, scn)
+        sv.set_fuse_sources(True)
+        sv.tune_sweeps(scn.dt, 10)
+        assert sv.get_fuse_sources() and sv.get_closed_sweep(0) == 0
+        sv.set_fuse_sources(False)
+        assert sv.get_closed_sweep(0) > 0

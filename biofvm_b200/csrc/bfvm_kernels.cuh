@@ -326,12 +326,18 @@ __device__ __forceinline__ bool div_safe(double x) {
 // (voxel, density) the chain index - field - store ran in seven waves of
 // blocks (0.5M voxels: x 4 FP64 13.8 -> 9.4 us, x 10 30.1 -> 16.6).
 constexpr int kBulkPerLane = 8;
+// The run a warp takes, eight warps to a block (at most 2^31 runs).  2^27 of
+// them make 2^32 threads, whose numbers do not fit 32 bits.
+__host__ __device__ constexpr uint32_t bulk_run(uint32_t block, uint32_t thread) {
+  return block * 8u + (thread >> 5);
+}
 template <typename T>
 __global__ void __launch_bounds__(256)
     bulk_runs_kernel(T* __restrict__ p, int S, int lanes, int nruns, const int4* __restrict__ runs,
                      const double* __restrict__ tab, double dt) {
-  const int w = (int)((blockIdx.x * 256u + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (w >= nruns || lane >= lanes) return;
+  const uint32_t w = bulk_run(blockIdx.x, threadIdx.x);
+  const int lane = threadIdx.x & 31;
+  if (w >= (uint32_t)nruns || lane >= lanes) return;
   const int4 run = __ldg(runs + w);
   const int count = run.y * S;
   T* q = p + (int64_t)run.x * S + lane;

@@ -930,12 +930,12 @@ std::string plan_key(const bfvm_batch* b, double dt, int nsteps, int flags) {
         k.push_back(L.present ? 1 : 0);
       };
       buf(m->p);
+      buf(m->closed_tab);
       for (int a = 0; a < 3; ++a) {
         buf(m->coef[a]);
         buf(m->chunk[a]);
         buf(m->chunk_il[a]);
         buf(m->chunk_slots[a]);
-        buf(m->closed_tab[a]);
       }
       for (const DevBuf* d : {&m->d_bulk_vox, &m->d_bulk_st, &m->d_bulk_su, &m->d_dir_vox,
                               &m->d_dir_val, &m->d_ag_vox_orig, &m->d_ag_t1, &m->d_ag_t2,

@@ -1636,13 +1636,13 @@ int bfvm_destroy(bfvm_solver* m) {
     m->d_status.release();
     m->d_grad.release();
     adjoint_release(m);
-    for (auto& c : m->closed_tab) c.release();
+    m->closed_tab.release();
     for (auto& c : m->chunk) c.release();
     for (auto& c : m->chunk_il) c.release();
     for (auto& c : m->chunk_slots) c.release();
     for (auto& c : m->cl_tab) c.release();
     m->d_grid_maps.release();
-    for (auto& c : m->grid_tab) c.release();
+    m->grid_tab.release();
     cudaStreamDestroy(m->stream);
     delete m;
   });
@@ -2345,10 +2345,9 @@ void grid_run(bfvm_solver* m, double dt, int nsteps, int flags, const GridPlan& 
   if (!m->grid_tab_ok) {
     std::vector<double> t;
     std::vector<float> tf;
-    for (int a = 0; a < 3; ++a) {
-      closed_constants(m, a, bfvm::kGridChunk, t, tf);
-      upload(m->grid_tab[a], t, m->stream);
-    }
+    const int ch[3] = {bfvm::kGridChunk, bfvm::kGridChunk, bfvm::kGridChunk};
+    closed_constants(m, ch, t, tf, m->grid_off);
+    upload(m->grid_tab, t, m->stream);
     m->grid_tab_ok = true;
   }
   // scratch: Dirichlet values [N][S] (doubles first), line masks of the x and
@@ -2399,7 +2398,7 @@ void grid_run(bfvm_solver* m, double dt, int nsteps, int flags, const GridPlan& 
   if (m->dir_unique > 0) a.on |= bfvm::kVoxDirichlet;
   const int ns[3] = {m->nx, m->ny, m->nz};
   for (int ax = 0; ax < 3; ++ax) {
-    a.cst[ax] = m->grid_tab[ax].as<double>();
+    a.cst[ax] = m->grid_tab.as<double>() + m->grid_off[ax];
     a.cst_count[ax] = (int)grid_constants(ns[ax], S);
   }
   a.staged = P.staged;

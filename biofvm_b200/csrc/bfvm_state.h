@@ -175,10 +175,11 @@ struct bfvm_solver {
   int chunk_ch[3] = {0, 0, 0};
   int chunk_nslots[3] = {0, 0, 0};
   bfvm_rt::Axis axis[3];
-  // constants of the closed-form sweeps per axis (cst [S][8], pw [chunks][S][2]),
-  // built with the Thomas setup; whether its coefficients have the closed
+  // constants of the closed-form sweeps (per axis, from closed_off: cst [S][8],
+  // pw [chunks][S][2]), built with the Thomas setup; whether its coefficients have the closed
   // form; lod_dims at that setup
-  bfvm_rt::DevBuf closed_tab[3];
+  bfvm_rt::DevBuf closed_tab;
+  size_t closed_off[3] = {0, 0, 0};
   bool closed_ok = true;
   int setup_dims = 3;
 
@@ -260,7 +261,8 @@ struct bfvm_solver {
   bool grid_tab_ok = false;
   int grid_resident = 0;  // blocks of the grid steps the device holds at grid_smem
   size_t grid_smem = 0;
-  bfvm_rt::DevBuf grid_tab[3];
+  bfvm_rt::DevBuf grid_tab;
+  size_t grid_off[3] = {0, 0, 0};
   // cached tensor maps of the line sweeps, per axis, with the geometry they
   // were encoded for (field address, element size, C, n, outer blocks, the
   // two strides, tile width, box rows): a resize that keeps the allocation,
@@ -331,8 +333,8 @@ void allow_smem(const void* kernel, int device, size_t bytes);
 bool closed_axis(const bfvm_solver* m, int ax);
 int closed_axis_chunk(const bfvm_solver* m, int ax);
 void closed_setup(bfvm_solver* m);
-void closed_constants(const bfvm_solver* m, int a, int ch, std::vector<double>& t,
-                      std::vector<float>& tf);
+void closed_constants(const bfvm_solver* m, const int (&ch)[3], std::vector<double>& t,
+                      std::vector<float>& tf, size_t (&off)[3]);
 void closed_sweep(bfvm_solver* m, int ax, int fuse, int64_t z0, int64_t z1);
 // Defined in bfvm_adjoint.cu.
 void adjoint_release(bfvm_solver* m);

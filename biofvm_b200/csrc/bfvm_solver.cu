@@ -350,7 +350,15 @@ void build_bulk(bfvm_solver* m) {
     const int64_t cap = std::max<int64_t>(1, E / 4);
     std::string key((size_t)S * 2 * sizeof(double), '\0');
     bool ok = true;
+    const size_t row_bytes = (size_t)S * sizeof(double);
     for (int64_t e = 0; e < E && ok; ++e) {
+      vox32[e] = (int)m->bulk_vox[e];
+      // a region's voxels share their row with the one before: no look-up
+      if (e > 0 && std::memcmp(&m->bulk_st[e * S], &m->bulk_st[(e - 1) * S], row_bytes) == 0 &&
+          std::memcmp(&m->bulk_su[e * S], &m->bulk_su[(e - 1) * S], row_bytes) == 0) {
+        row[e] = row[e - 1];
+        continue;
+      }
       for (int s = 0; s < S; ++s) {
         std::memcpy(&key[(size_t)s * 2 * sizeof(double)], &m->bulk_st[e * S + s], sizeof(double));
         std::memcpy(&key[((size_t)s * 2 + 1) * sizeof(double)], &m->bulk_su[e * S + s],
@@ -369,7 +377,6 @@ void build_bulk(bfvm_solver* m) {
         }
       }
       row[e] = it->second;
-      vox32[e] = (int)m->bulk_vox[e];
     }
     if (ok) {
       upload(m->d_bulk_vox32, vox32, st);

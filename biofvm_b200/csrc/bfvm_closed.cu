@@ -24,12 +24,15 @@ int axis_points(const bfvm_solver* m, int a) { return a == 0 ? m->nx : (a == 1 ?
 // us, at 256^3 x 4 FP32 132 -> 98), but a line's last, partial chunk runs the
 // body with bounds checks, a quarter of the threads of a 123-point line (z at
 // 161 x 97 x 123 x 3: 20.2 us at 16 points, 22.9 at 32).
-// Fields of few columns take 16 as well, to have threads on every SM (twelve
-// domains of 32 to 128 points a side, 20 steps: 4.19 -> 4.07 ms).
+// Fields of few columns take 16 as well, to have 128 threads on every SM
+// (twelve domains of 32 to 128 points a side, 20 steps: 4.19 -> 4.07 ms).  The
+// columns are counted over the whole mesh, also where LOD_2D sweeps one plane
+// of a mesh with several: the constants are laid out for one chunk length,
+// which may not change between a 3-D and a 2-D step.
 int closed_chunk(const bfvm_solver* m, int a) {
   const int n = axis_points(m, a);
   if (n > 512) return 32;
-  if (m->NS() / n * ((n + 31) / 32) < 128 * 148) return 16;
+  if (m->NS() / n * ((n + 31) / 32) < 128 * (int64_t)m->num_sms) return 16;
   return n % 32 == 0 || n > 160 ? 32 : 16;
 }
 

@@ -2,9 +2,9 @@
 //
 // A field of up to 2^19 voxel-densities with at most 64 points per axis costs
 // more in kernel start-up than in work when every phase of a step is its own
-// launch.  Here every step runs inside one launch, as two phases separated by
-// grid-wide barriers of a cooperative launch (all blocks are resident, so each
-// barrier completes):
+// launch.  Here every step runs inside one launch, as two phases (or three,
+// below) separated by grid-wide barriers of a cooperative launch (all blocks are
+// resident, so each barrier completes):
 //   xy: an item is one xy plane (of sg of its densities), held in shared
 //       memory.  As it is loaded, its voxels take the bulk update
 //       (BioFVM_microenvironment.cpp:603-609), then their agents in list order
@@ -23,12 +23,14 @@
 // grid barrier also empties L1, so that anything read again after it costs an
 // L2 round trip: the lines' constants are copied to shared memory once, and a
 // plane's loads are two rounds (the field with the maps, then what they point
-// to).  One block per SM: with two, the registers spill (50^3 x 4 22.7 ->
-// 32.7 us).  Steps of 50^3 x 1 with 1000 agents and a fixed boundary, 100 in a
-// call: 13.2 us, of three solvers at once 6.7 a step (16.9 and 9.9 with three
-// phases x, y, z through memory and the elimination's per-point tables); 24^3
-// x 20 14.1 (18.5), 32^3 x 8 12.9 (14.9), 64^3 x 2 16.1 (22.4), 50^3 x 4, with
-// more planes than SMs, 23.7 (22.5).
+// to).  One block per SM: with two, the registers spill.  Steps with 1000
+// agents and a fixed boundary, 100 in a call, in us (in brackets with three
+// phases x, y, z through memory and the elimination's per-point tables): 50^3 x
+// 1 13.1 (16.8), of three solvers at once 6.7 a step (9.9); 24^3 x 20 14.0
+// (18.3), 32^3 x 8 13.1 (14.9), 64^3 x 2 16.0 (22.4), 64 x 64 x 16 x 1 15.9
+// (15.3; of three at once 5.7, 6.2).  Three solvers at once with planes for 75
+// to 148 blocks each find no SMs beside one another: 32^3 x 3, calls of one
+// step, 8.9 -> 11.7 a step, where one alone takes 21.4 -> 15.3.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -57,6 +59,10 @@ struct GridStepArgs {
   int tw;               // columns of a z tile: tw x chunks of nz <= kGridThreads
   uint64_t m_sg, m_last, m_nx;  // quot() of sg, of the last item's, of nx,
   uint64_t m_lx, m_ly, m_lx_last, m_ly_last, m_tw;  // of an item's x and y lines, of tw
+  // a phase per axis: its columns, the columns of a tile; quot() of those, S, nx S
+  bool first;  // the first step's sources in a pass of their own
+  int pcols[3], ptw[3];
+  uint64_t m_ptw[3], m_S, m_rowS;
   const unsigned char* flags;   // [N]
   // per flagged voxel: its bulk entry; its first agent's place in the sorted
   // list and in the agent list
@@ -279,6 +285,202 @@ static __global__ void __launch_bounds__(kGridThreads, 1) grid_steps_kernel(cons
       __syncthreads();
     }
     if (step + 1 < a.nsteps) grid.sync();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The same steps with a phase per axis, every line straight from and to the
+// field: a block takes tw columns x chunks of the axis.  The sources and
+// Dirichlet values of a step are applied as the z phase before it stores its
+// points, the first step's as its x lines load.  At a node the x and y lines
+// store nothing, so its value stays through both.  UPD: the steps have any of
+// them.
+//
+// A barrier more a step, but the work splits finer than whole planes: for few
+// wide planes, where a thread of the planes' blocks takes up to eight voxels'
+// source chains (64 x 64 x 1 with 1000 agents and bulk rates 21.6 -> 13.6 us a
+// step), and for more planes than SMs, whose second wave is mostly empty
+// (50^3 x 4 with the same sources 28.2 -> 17.8, without 19.5 -> 13.6).  With
+// 1000 agents and a fixed boundary, 100 steps in a call: 50^3 x 4 23.6 -> 15.1
+// (22.7 with the three phases and tables mentioned above), 43^3 x 6 22.6 -> 15.2
+// (22.1), 64 x 64 x 2 x 20 24.8 -> 14.8 (17.8), 64 x 64 x 1 x 1 18.7 -> 12.7 (12.4).
+// bfvm_solver.cu's grid_phases_better has the rule.
+
+constexpr int kPhaseThreads = 256;
+template <int AX>
+struct Axis3 {
+  static constexpr int value = AX;
+};
+
+// Sources and Dirichlet values of a thread's points of one line: vox0 the voxel
+// of its first point, vstep between points.  The points' maps come in one
+// round trip.  Agents after a voxel's first one follow in a loop of their own,
+// in which a lane goes on to its next such point without waiting for the
+// warp's others.  (Fetching every constant of four points at once spills, and
+// is slower everywhere: 64 x 64 x 2 x 4 14.1 -> 15.7 us a step.)
+__device__ __forceinline__ void grid_update(const GridStepArgs& a, double (&x)[kGridChunk], int len,
+                                            int vox0, int vstep, int s) {
+  int f[kGridChunk], be[kGridChunk], ag[kGridChunk];
+#pragma unroll
+  for (int m = 0; m < kGridChunk; ++m) {
+    const int vox = vox0 + m * vstep;
+    f[m] = m < len ? __ldg(a.flags + vox) : 0;
+    if (m < len && (a.on & kVoxBulk)) be[m] = __ldg(a.bulk_map + vox);
+    if (m < len && (a.on & kVoxAgents)) ag[m] = __ldg(&a.ag_map[vox].y);
+  }
+  unsigned more = 0;
+#pragma unroll
+  for (int m = 0; m < kGridChunk; ++m) {
+    const int flags = f[m] & a.on;
+    if (flags & kVoxDirichlet) {
+      x[m] = __ldg(a.dir_field + (int64_t)(vox0 + m * vstep) * a.S + s);
+    } else if (flags) {
+      if (flags & kVoxBulk) {
+        const int64_t e = (int64_t)be[m] * a.S + s;
+        x[m] = bulk_update(x[m], __ldg(a.bulk_st + e), __ldg(a.bulk_su + e), a.dt);
+      }
+      if (flags & kVoxAgents) {
+        const int64_t e = (int64_t)ag[m] * a.S + s;
+        x[m] = cell_update(x[m], __ldg(a.ag_t1 + e), __ldg(a.ag_t2 + e));
+        if (f[m] & kVoxMoreAgents) more |= 1u << m;
+      }
+    }
+  }
+  int m = -1, r = 0;
+  uint64_t vox = 0;
+  double v = 0.0;
+  while (m >= 0 || more) {
+    if (m < 0) {
+      m = __ffs(more) - 1;
+      more &= more - 1;
+      vox = (uint64_t)(vox0 + m * vstep);
+      r = __ldg(&a.ag_map[vox].x) + 1;
+      v = reg_get<double, kGridChunk>(x, m);
+    }
+    const int64_t e = (int64_t)__ldg(a.ag_idx + r) * a.S + s;
+    const bool last = r + 1 >= a.nagents || __ldg(a.ag_key + r + 1) != vox;
+    v = cell_update(v, __ldg(a.ag_t1 + e), __ldg(a.ag_t2 + e));
+    ++r;
+    if (last) {
+      reg_set<double, kGridChunk>(x, m, v);
+      m = -1;
+    }
+  }
+}
+
+// The same for the whole field, an element per thread: with few elements to a
+// thread shorter than eight in a row, though it takes a barrier more.
+__device__ __forceinline__ void grid_update_first(const GridStepArgs& a) {
+  const int count = a.nx * a.ny * a.nz * a.S;
+  for (int w = blockIdx.x * kPhaseThreads + threadIdx.x; w < count;
+       w += gridDim.x * kPhaseThreads) {
+    const int vox = (int)quot(w, a.m_S), s = w - vox * a.S;
+    const int flags = __ldg(a.flags + vox) & (a.on | kVoxMoreAgents);
+    if (!(flags & a.on)) continue;
+    double x = a.p[w];
+    if (flags & kVoxDirichlet) {
+      x = __ldg(a.dir_field + w);
+    } else {
+      if (flags & kVoxBulk) {
+        const int64_t e = (int64_t)__ldg(a.bulk_map + vox) * a.S + s;
+        x = bulk_update(x, __ldg(a.bulk_st + e), __ldg(a.bulk_su + e), a.dt);
+      }
+      if (flags & kVoxAgents) {
+        const int2 first = __ldg(a.ag_map + vox);
+        int64_t e = (int64_t)first.y * a.S + s;
+        x = cell_update(x, __ldg(a.ag_t1 + e), __ldg(a.ag_t2 + e));
+        if (flags & kVoxMoreAgents)
+          for (int r = first.x + 1; r < a.nagents && __ldg(a.ag_key + r) == (uint64_t)vox; ++r) {
+            e = (int64_t)__ldg(a.ag_idx + r) * a.S + s;
+            x = cell_update(x, __ldg(a.ag_t1 + e), __ldg(a.ag_t2 + e));
+          }
+      }
+    }
+    a.p[w] = x;
+  }
+}
+
+template <int AX, bool UPD>
+__device__ __forceinline__ void grid_lines(const GridStepArgs& a, int tile, const double* cst,
+                                           bool update, double* sU, double* sW) {
+  const int S = a.S, plane = a.nx * a.ny, n = AX == 0 ? a.nx : (AX == 1 ? a.ny : a.nz);
+  const int ncols = a.pcols[AX], TW = a.ptw[AX], NC = (n + kGridChunk - 1) / kGridChunk;
+  const int c = (int)quot(threadIdx.x, a.m_ptw[AX]), tx = threadIdx.x - c * TW;
+  const int col = tile * TW + tx, vcol = min(col, ncols - 1);
+  const int len = c < NC && col < ncols ? min(kGridChunk, n - c * kGridChunk) : 0;
+  const int l = (int)quot(vcol, a.m_S), s = vcol - l * S;  // line (k, j), (k, i) or (j, i)
+  int64_t off;     // of the line's first point
+  int ls;          // between its points
+  int vox0, vstep; // voxels likewise
+  if (AX == 0) {
+    off = (int64_t)l * a.nx * S + s, ls = S, vox0 = l * a.nx, vstep = 1;
+  } else if (AX == 1) {
+    const int k = (int)quot(vcol, a.m_rowS), in = vcol - k * a.nx * S;
+    off = (int64_t)k * plane * S + in, ls = a.nx * S, vox0 = 0, vstep = 0;
+  } else {
+    off = vcol, ls = plane * S, vox0 = l, vstep = plane;
+  }
+  const int k0 = c * kGridChunk;
+  unsigned nodes = 0;
+  if (UPD && AX < 2 && (a.on & kVoxDirichlet) && len > 0)
+    nodes = (unsigned)(__ldg((AX == 0 ? a.dir_mask_x : a.dir_mask_y) + l) >> k0) & 0xffu;
+  double* q = a.p + off + (int64_t)k0 * ls;
+  double v[kGridChunk];
+#pragma unroll
+  for (int m = 0; m < kGridChunk; ++m)
+    v[m] = m < len ? (AX == 0 ? q[m * ls] : __ldcg(q + m * ls)) : 0.0;
+  if (UPD && AX == 0 && update) {
+    grid_update(a, v, len, vox0 + k0 * vstep, vstep, s);
+#pragma unroll
+    for (int m = 0; m < kGridChunk; ++m)
+      if (nodes >> m & 1u) q[m * ls] = v[m];
+  }
+  grid_chunk(v, len, cst, S, s, sU, sW, TW, NC, c, tx);
+  if (UPD && AX == 2 && update) grid_update(a, v, len, vox0 + k0 * vstep, vstep, s);
+#pragma unroll
+  for (int m = 0; m < kGridChunk; ++m)
+    if (m < len && !(nodes >> m & 1u)) q[m * ls] = v[m];
+}
+
+template <bool UPD>
+__global__ void __launch_bounds__(kPhaseThreads, 2)
+    grid_phases_kernel(const GridStepArgs a) {
+  namespace cg = cooperative_groups;
+  cg::grid_group grid = cg::this_grid();
+  extern __shared__ __align__(16) double grid_smem[];
+  double* sU = grid_smem;
+  double* sW = sU + kPhaseThreads;
+  const double* cst[3] = {a.cst[0], a.cst[1], a.cst[2]};
+  if (a.staged) {
+    double* t = grid_smem + 2 * kPhaseThreads;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+      for (int i = threadIdx.x; i < a.cst_count[ax]; i += kPhaseThreads) t[i] = __ldg(cst[ax] + i);
+      cst[ax] = t;
+      t += a.cst_count[ax];
+    }
+    __syncthreads();
+  }
+  auto phase = [&](auto ax, bool update) {
+    constexpr int AX = decltype(ax)::value;
+    const int tiles = (a.pcols[AX] + a.ptw[AX] - 1) / a.ptw[AX];
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+      grid_lines<AX, UPD>(a, t, cst[AX], update, sU, sW);
+      __syncthreads();  // the fold is free again
+    }
+  };
+  if (UPD && a.first) {
+    grid_update_first(a);
+    grid.sync();
+  }
+  for (int step = 0; step < a.nsteps; ++step) {
+    const bool more = step + 1 < a.nsteps;
+    phase(Axis3<0>(), a.on && step == 0 && !a.first);
+    grid.sync();
+    phase(Axis3<1>(), false);
+    grid.sync();
+    phase(Axis3<2>(), a.on && more);
+    if (more) grid.sync();
   }
 }
 

@@ -2279,8 +2279,8 @@ void cluster_run(bfvm_solver* m, double dt, int nsteps, int flags, int cl) {
 }
 
 constexpr int kGridMaxN = 64;  // points per axis (8-point chunks, 8 of them)
-// voxel-densities: at 64^3 x 2 = 2^19 15.9 us a step against 29.6 with the
-// sweep kernels, at 50^3 x 4 22.8 against 28.7
+// voxel-densities: at 64^3 x 2 = 2^19 16.0 us a step against 28.7 with the
+// sweep kernels, at 50^3 x 4 15.1 against 28.7
 constexpr int64_t kGridMaxVS = 1 << 19;
 
 constexpr size_t kGridSmemMost = 200 * 1024;
@@ -2292,14 +2292,39 @@ size_t grid_constants(int n, int S) {
 
 struct GridPlan {
   int blocks = 0;  // 0: bfvm_step does not take the grid steps
-  int sg = 0, groups = 0, pitch = 0;
-  int tw = 0;
+  bool phases = false;  // a phase per axis (grid_phases_kernel)
+  bool first = false;   // its first sources in a pass of their own
+  int sg = 0, groups = 0, pitch = 0, tw = 0;  // grid_steps_kernel
+  int ptw[3] = {0, 0, 0};                     // grid_phases_kernel: columns per tile
   bool staged = false;  // the lines' constants in shared memory
   size_t smem = 0;
+  const void* kernel = nullptr;
+  int threads = 0;
 };
 
+// Whether a phase per axis is faster than xy planes (`groups` items of sg
+// densities per plane).  From steps of 565 shapes of 8 to 64 points a side, 1 to
+// 64 planes and 1 to 20 densities on 148 SMs, the time of the xy planes over
+// that of the phases, without sources / with 500 agents and nodes / with 1000
+// agents, nodes and bulk rates:
+//   more items than SMs: 1.36 / 1.50 / 1.55;
+//   planes of 3000 elements or more: up to 20 items 1.13 / 1.48 / 1.62, to 40
+//     1.14 / 1.32 / 1.36;
+//   1700 to 3000 elements, up to 20 items: 0.98 / 1.22 / 1.30, but from 8
+//     planes on up to 1.15 times slower in calls of one step;
+//   fewer: 0.91 / 0.90 / 0.84.
+// With 41 to 80 items of 1700 elements or more the phases are ahead as well,
+// but not for calls of one step by solvers side by side, which find fewer SMs
+// free (three of 50^3 x 1: 5.9 -> 6.8 us).
+bool grid_phases_better(const bfvm_solver* m, int sg, int groups, bool sources) {
+  const int items = m->nz * groups, plane = m->nx * m->ny * sg;
+  if (items > m->num_sms) return true;
+  if (7 * items > (sources ? 2 : 1) * m->num_sms) return false;
+  return plane >= 3000 ? m->nz <= 8 : sources && plane >= 1700 && m->nz <= 4;
+}
+
 // The cooperative launch that runs this solver's steps in one launch.
-GridPlan plan_grid(bfvm_solver* m) {
+GridPlan plan_grid(bfvm_solver* m, int flags) {
   GridPlan P;
   if (!m->grid_steps || m->path != BFVM_PATH_AUTO || m->precision != BFVM_FP64 ||
       m->lod_dims != 3 || !m->uniform || m->fuse_sources || m->slab_planes > 0 ||
@@ -2315,9 +2340,19 @@ GridPlan plan_grid(bfvm_solver* m) {
   P.groups = std::max((m->S + P.sg - 1) / P.sg, std::min(m->S, m->num_sms / m->nz));
   P.sg = (m->S + P.groups - 1) / P.groups;
   P.groups = (m->S + P.sg - 1) / P.sg;
+  const bool sources = !m->dir_vox.empty() ||
+                       ((flags & BFVM_STEP_BULK) && !m->bulk_vox.empty()) ||
+                       ((flags & BFVM_STEP_CELLS) && m->n_agents > 0);
+  const bool phases = grid_phases_better(m, P.sg, P.groups, sources);
   const int width = m->nx * P.sg;
   P.pitch = width + ((P.sg - width) % 16 + 16) % 16;
-  size_t doubles = bfvm::grid_smem_doubles(m->ny, P.pitch);
+  P.phases = phases;
+  P.kernel = !phases   ? (const void*)bfvm::grid_steps_kernel
+             : sources ? (const void*)bfvm::grid_phases_kernel<true>
+                       : (const void*)bfvm::grid_phases_kernel<false>;
+  P.threads = phases ? bfvm::kPhaseThreads : bfvm::kGridThreads;
+  size_t doubles =
+      phases ? 2 * bfvm::kPhaseThreads : bfvm::grid_smem_doubles(m->ny, P.pitch);
   size_t consts = 0;
   for (int n : {m->nx, m->ny, m->nz}) consts += grid_constants(n, m->S);
   P.staged = (doubles + consts) * sizeof(double) <= kGridSmemMost;
@@ -2329,20 +2364,40 @@ GridPlan plan_grid(bfvm_solver* m) {
   const int cz = (m->nz + bfvm::kGridChunk - 1) / bfvm::kGridChunk;
   const int64_t tiles = 32 * std::max<int64_t>((int64_t)m->nz * P.groups, 32);
   P.tw = (int)std::min<int64_t>(bfvm::kGridThreads / cz / 32 * 32, (cols + tiles - 1) / tiles * 32);
-  const int64_t work = std::max<int64_t>((int64_t)m->nz * P.groups, blocks_for(cols, P.tw));
-  if (m->grid_smem != P.smem) {
-    const void* k = (const void*)bfvm::grid_steps_kernel;
+  int64_t work = std::max<int64_t>((int64_t)m->nz * P.groups, blocks_for(cols, P.tw));
+  const int most = phases ? 2 : 1;  // blocks per SM
+  if (phases) {
+    // half as many tiles as SMs, of a warp's columns or more, as far as a
+    // block's threads reach: a tile per SM is no faster (64 x 64 x 4 x 1 12.2
+    // and 12.2 us a step) and leaves solvers side by side less room (calls of
+    // one step by three of them 8.6 -> 6.9 us)
+    work = 1;
+    const int ns[3] = {m->nx, m->ny, m->nz};
+    for (int a = 0; a < 3; ++a) {
+      const int nc = (ns[a] + bfvm::kGridChunk - 1) / bfvm::kGridChunk;
+      const int64_t c = m->NS() / ns[a];
+      P.ptw[a] = (int)std::min<int64_t>(P.threads / nc,
+                                        std::max<int64_t>(32, blocks_for(c, m->num_sms / 2)));
+      work = std::max(work, blocks_for(c, P.ptw[a]));
+    }
+  }
+  if (m->grid_smem != P.smem || m->grid_kernel != P.kernel) {
+    const void* k = P.kernel;
     int coop = 0, per_sm = 0;
     BFVM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->device));
     if (coop) {
       allow_smem(k, m->device, P.smem);
       BFVM_CUDA(
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, bfvm::kGridThreads, P.smem));
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, P.threads, P.smem));
     }
-    m->grid_resident = std::min(per_sm, 1) * m->num_sms;
+    m->grid_resident = std::min(per_sm, most) * m->num_sms;
     m->grid_smem = P.smem;
+    m->grid_kernel = k;
   }
   P.blocks = (int)std::min<int64_t>(work, m->grid_resident);
+  // up to two elements a thread: 64 x 64 x 1 x 1 with sources, calls of one
+  // step, 23.4 -> 19.3 us; 64 x 64 x 2 x 20, at 4.3, 21.5 -> 23.4
+  P.first = phases && m->NS() <= 2 * (int64_t)P.blocks * P.threads;
   return P;
 }
 
@@ -2422,6 +2477,16 @@ void grid_run(bfvm_solver* m, double dt, int nsteps, int flags, const GridPlan& 
   a.m_lx_last = quot_of((uint64_t)m->ny * last);
   a.m_ly_last = quot_of((uint64_t)m->nx * last);
   a.m_tw = quot_of(P.tw);
+  if (P.phases) {
+    a.first = P.first;
+    for (int ax = 0; ax < 3; ++ax) {
+      a.pcols[ax] = (int)(m->NS() / ns[ax]);
+      a.ptw[ax] = P.ptw[ax];
+      a.m_ptw[ax] = quot_of(P.ptw[ax]);
+    }
+    a.m_S = quot_of(S);
+    a.m_rowS = quot_of((uint64_t)m->nx * S);
+  }
   a.flags = vox_flags;
   a.bulk_map = bulk_map;
   a.ag_map = ag_map;
@@ -2436,8 +2501,8 @@ void grid_run(bfvm_solver* m, double dt, int nsteps, int flags, const GridPlan& 
   a.ag_t1 = m->d_ag_t1.as<double>();
   a.ag_t2 = m->d_ag_t2.as<double>();
   void* params[] = {&a};
-  BFVM_CUDA(cudaLaunchCooperativeKernel((const void*)bfvm::grid_steps_kernel, dim3((unsigned)P.blocks),
-                                        dim3(bfvm::kGridThreads), params, P.smem, m->stream));
+  BFVM_CUDA(cudaLaunchCooperativeKernel(P.kernel, dim3((unsigned)P.blocks),
+                                        dim3((unsigned)P.threads), params, P.smem, m->stream));
   check_launch(m);
 }
 
@@ -2450,7 +2515,7 @@ int bfvm_set_grid_steps(bfvm_solver* m, int enable) {
 int bfvm_get_grid_steps(bfvm_solver* m, int* blocks) {
   return SOLVER_CALL(m, {
     require(blocks != nullptr, "null output pointer");
-    *blocks = plan_grid(m).blocks;
+    *blocks = plan_grid(m, BFVM_STEP_ALL).blocks;
   });
 }
 
@@ -2494,7 +2559,7 @@ int bfvm_step(bfvm_solver* m, double dt, int nsteps, int flags) {
       check_lod_mesh(m);
       thomas_setup(m, dt);
     }
-    const GridPlan grid = nsteps > 0 ? plan_grid(m) : GridPlan();
+    const GridPlan grid = nsteps > 0 ? plan_grid(m, flags) : GridPlan();
     if (grid.blocks > 0) {
       check_lod_mesh(m);
       build_all(m);

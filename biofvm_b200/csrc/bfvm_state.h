@@ -259,8 +259,9 @@ struct bfvm_solver {
   // constants of the three axes for the grid steps' 8-point chunks, rebuilt
   // after each Thomas setup
   bool grid_tab_ok = false;
-  int grid_resident = 0;  // blocks of the grid steps the device holds at grid_smem
+  int grid_resident = 0;  // blocks of grid_kernel the device holds at grid_smem
   size_t grid_smem = 0;
+  const void* grid_kernel = nullptr;
   bfvm_rt::DevBuf grid_tab;
   size_t grid_off[3] = {0, 0, 0};
   // cached tensor maps of the line sweeps, per axis, with the geometry they

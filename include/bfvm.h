@@ -350,8 +350,9 @@ BFVM_API int bfvm_get_cluster_steps(bfvm_solver* m, int* blocks);
  * points (and the cluster mode above is not in use).  Each step is two phases
  * separated by grid-wide barriers: xy planes in shared memory (bulk and cell
  * updates and Dirichlet values as they load, then the x and y lines), and
- * tiles of z columns.  On by default (15.9 vs 29.6 us per step at 64^3 x 2 on
- * a B200, 22.8 vs 28.7 at 50^3 x 4); enable = 0 gives back the sweep
+ * tiles of z columns; for few wide planes and for more planes than SMs three,
+ * x, y and z lines.  On by default (16.0 vs 28.7 us per step at 64^3 x 2 on
+ * a B200, 15.1 vs 28.7 at 50^3 x 4); enable = 0 gives back the sweep
  * kernels.  bfvm_get_grid_steps gives the launch's block count for this
  * solver now (0: not used). */
 BFVM_API int bfvm_set_grid_steps(bfvm_solver* m, int enable);

@@ -807,6 +807,9 @@ LinesPlan plan_lines(const bfvm_solver* m, int ax) {
   if (ax == 0 && L.C % L.w) return L;  // x: whole tiles of densities only
   L.box_n = std::min(L.n, 256);
   L.nboxes = (L.n + L.box_n - 1) / L.box_n;
+  // a tile starts on a 128-byte boundary, as its copy must (an FP32 field in
+  // FP64 arithmetic has rows of 64 bytes: an odd number of them is made even)
+  while ((L.box_n * L.w * es) % 128) ++L.box_n;
   const int64_t ctiles = (L.C + L.w - 1) / L.w;
   if (ctiles * L.nouter >= ((int64_t)1 << 31)) return L;
   const size_t stage = (size_t)L.box_n * L.nboxes * L.w * es;

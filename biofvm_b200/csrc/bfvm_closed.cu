@@ -18,12 +18,28 @@ namespace {
 
 int axis_points(const bfvm_solver* m, int a) { return a == 0 ? m->nx : (a == 1 ? m->ny : m->nz); }
 
-// Points per thread: 32 where the line is whole 32-point chunks or has at
-// least six of them, else 16.  A 32-point chunk spreads the per-thread work
-// (indices, carries) over twice the points (y at 256^3 x 10 FP64 415 -> 396
-// us, at 256^3 x 4 FP32 132 -> 98), but a line's last, partial chunk runs the
-// body with bounds checks, a quarter of the threads of a 123-point line (z at
-// 161 x 97 x 123 x 3: 20.2 us at 16 points, 22.9 at 32).
+// Whether a short line takes chunks of 8 points: a thread's passes are unrolled
+// over its chunk, and along x, where a chunk's loads touch a few bytes of each
+// sector, fewer of them help by themselves.  Sweeps of 12M elements in us, with
+// 16-point chunks -> with 8: lines of 3, FP64 x of one density 42 -> 22, FP32 y of
+// four 80 -> 51; of 12, x of one FP64 79 -> 62, FP32 60 -> 32, y FP64 38.9 -> 38.6,
+// FP32 24.5 -> 29.6 (16 kept); of 9, y FP64 34.8 -> 37.4 (16 kept), x of ten FP32
+// 31.4 -> 39.3 (16 kept from three on); of 16, y FP64 26.6 -> 28.6 (16 kept); of
+// 20, x of one FP64 88 -> 76, FP32 62 -> 44; of 30, x FP64 of one 81 -> 76, of two
+// 43 -> 46 (16 kept).
+bool closed_short(const bfvm_solver* m, int a) {
+  const int n = axis_points(m, a);
+  if (n <= 8) return true;
+  if (n == 16 || (m->math_elem() == 4 && (a != 0 || m->S > 2))) return false;
+  return n <= 24 ? a == 0 || n >= 12 : a == 0 && n < 32 && m->S == 1;
+}
+
+// Points per thread: 8 for short lines (above); 32 where the line is whole
+// 32-point chunks or has at least six of them; else 16.  A 32-point chunk
+// spreads the per-thread work (indices, carries) over twice the points (y at
+// 256^3 x 10 FP64 415 -> 396 us, at 256^3 x 4 FP32 132 -> 98), but a line's last,
+// partial chunk runs the body with bounds checks, a quarter of the threads of a
+// 123-point line (z at 161 x 97 x 123 x 3: 20.2 us at 16 points, 22.9 at 32).
 // Fields of few columns take 16 as well, to have 128 threads on every SM
 // (twelve domains of 32 to 128 points a side, 20 steps: 4.19 -> 4.07 ms).  The
 // columns are counted over the whole mesh, also where LOD_2D sweeps one plane
@@ -31,6 +47,7 @@ int axis_points(const bfvm_solver* m, int a) { return a == 0 ? m->nx : (a == 1 ?
 // which may not change between a 3-D and a 2-D step.
 int closed_chunk(const bfvm_solver* m, int a) {
   const int n = axis_points(m, a);
+  if (closed_short(m, a)) return 8;
   if (n > 512) return 32;
   if (m->NS() / n * ((n + 31) / 32) < 128 * (int64_t)m->num_sms) return 16;
   return n % 32 == 0 || n > 160 ? 32 : 16;
@@ -216,11 +233,19 @@ void sweep_lines(bfvm_solver* m, int ax, int fuse, int64_t z0, int64_t z1) {
   if (ax == 2 || !dseg.present) fuse = 0;
   a.fuse = fuse & (bfvm::kFuseDirPro | bfvm::kFuseDirEpi);
   a.dir = dseg.view();
-  const int W = nc <= 16 ? 32 : 16;
+  // short lines: blocks of 64 threads, FP32 fields 128 (lines of 8 points, FP64
+  // y of one density 24.6 -> 20.3 us, FP32 24.4 -> 15.3; of 30, FP64 32.8 -> 34.5
+  // with 128, FP32 22.5 -> 21)
+  int W = nc <= 16 ? 32 : 16;
+  while (W * nc <= (sizeof(T) == 8 ? 32 : 64) &&
+         blocks_for(a.ncols - a.col0, 2 * W) >= 8 * m->num_sms)
+    W *= 2;
   const dim3 block(W, nc), grid((unsigned)blocks_for(a.ncols - a.col0, W));
   const size_t smem = (size_t)2 * nc * W * sizeof(CT);
   const bool ca = ax == 0 && S * (int)sizeof(T) < 256;
-  if (ch == 16)
+  if (ch == 8)
+    lines<T, CT, 8, 512>(m, a, ca, grid, block, smem);
+  else if (ch == 16)
     lines<T, CT, 16, 512>(m, a, ca, grid, block, smem);
   else if (W * nc <= 256)
     lines<T, CT, 32, 256>(m, a, ca, grid, block, smem);
@@ -241,7 +266,10 @@ struct TilePlan {
 };
 
 // The ring of an axis's tiles: 32 columns by n points each, 16 from 257 points
-// on, which keeps two blocks of 256 threads per SM up to 512 points.
+// on, which keeps two blocks of 256 threads per SM up to 512 points; FP32
+// fields' y and z from 513 points on, where 32 columns of 32-point chunks are
+// more than a block's threads (mixed, 12M elements in lines of 700: 42 -> 31 us
+// with tiles, FP32 28 -> 26.6).
 template <typename T, typename CT>
 TilePlan plan_tiles(const bfvm_solver* m, int ax, int64_t z0, int64_t z1) {
   TilePlan P;
@@ -250,7 +278,9 @@ TilePlan plan_tiles(const bfvm_solver* m, int ax, int64_t z0, int64_t z1) {
   const int n = axis_points(m, ax);
   P.ch = closed_chunk(m, ax);
   P.nc = (n + P.ch - 1) / P.ch;
-  const int W = P.w = P.ch == 32 && P.nc > 8 && (es == 8 || ax == 0) ? 16 : 32;
+  if (P.ch == 8) return P;  // the line kernel's
+  const int W = P.w =
+      P.ch == 32 && ((P.nc > 8 && (es == 8 || ax == 0)) || P.nc > 16) ? 16 : 32;
   P.maxt = P.ch == 16 || W * P.nc > 256 ? 512 : 256;
   if (W * P.nc > P.maxt) return P;
   if (ax == 0) {

@@ -213,7 +213,7 @@ __device__ __forceinline__ void closed_finish(CT (&v)[CH], int len, CT r, const 
 }
 
 // Blocks per SM the kernels are compiled for, from the registers a chunk of
-// CH points takes: FP64 64 of 65,536 / (512 x 2) at 16 points and 128 at 32;
+// CH points takes: FP64 64 of 65,536 / (512 x 2) up to 16 points and 128 at 32;
 // FP32 80 (three blocks of 256 threads) or 64 (two of 512) at 32 points.
 template <typename CT>
 constexpr int closed_min_blocks(int ch, int maxt) {

@@ -384,7 +384,10 @@ void build_bulk(bfvm_solver* m) {
       upload(m->d_bulk_tab, tab, st);
       m->bulk_rows = (int64_t)seen.size();
       // runs of consecutive voxels with one row, as long as a warp takes;
-      // worth it where they fill half of one on average
+      // worth it where they hold 96 elements on average: a warp takes a run
+      // whatever its length (0.5M listed voxels of 1M, time by voxels over
+      // time by runs: x 4 FP64 16 elements a run 0.34, 64 0.91, 96 1.14, 256
+      // 1.64; x 1 64 0.88, 128 1.34; x 20 60 0.87, 120 1.35)
       m->bulk_runs = 0;
       if (S <= 32) {
         const int most = std::max(1, 32 / S * bfvm::kBulkPerLane);
@@ -397,7 +400,7 @@ void build_bulk(bfvm_solver* m) {
           e = f;
         }
         const int64_t n = (int64_t)runs.size() / 4;
-        if (E * S >= 16 * n) {
+        if (E * S >= 96 * n) {
           upload(m->d_bulk_runs, runs, st);
           m->bulk_runs = n;
         }

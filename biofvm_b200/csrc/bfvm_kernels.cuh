@@ -529,6 +529,33 @@ __device__ __forceinline__ void gradient_rows_body(const GradArgs& a, const T* _
   }
 }
 
+// The same differences a row at a time, for meshes with too few rows to keep
+// the device busy four at a time: block (bx, j, k) covers 256 consecutive (i, s)
+// elements of row (j, k), whose results are staged in shared memory.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    gradient_row_kernel(const T* __restrict__ p, const GradArgs a) {
+  __shared__ double buf[3 * 256];
+  const int64_t RS = a.RS, e0 = (int64_t)blockIdx.x * 256, e = e0 + threadIdx.x;
+  const int count = (int)min((int64_t)256, RS - e0), j = blockIdx.y, k = blockIdx.z;
+  const int64_t row0 = ((int64_t)k * a.ny + j) * RS, jz = RS * a.ny;
+  double* out = a.g + 3 * (row0 + e0);
+  if (threadIdx.x < count) {
+    const T* q = p + row0 + e;
+    const double* old = out + 3 * threadIdx.x;
+    double* b = buf + 3 * threadIdx.x;
+    b[0] = e >= a.S && e + a.S < RS
+               ? __ddiv_rn(__dsub_rn((double)q[a.S], (double)q[-a.S]), a.dx.d)
+               : old[0];
+    b[1] = j > 0 && j < a.ny - 1 ? __ddiv_rn(__dsub_rn((double)q[RS], (double)q[-RS]), a.dy.d)
+                                 : old[1];
+    b[2] = k > 0 && k < a.nz - 1 ? __ddiv_rn(__dsub_rn((double)q[jz], (double)q[-jz]), a.dz.d)
+                                 : old[2];
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < 3 * count; c += 256) out[c] = buf[c];
+}
+
 template <typename T, bool FAST>
 __global__ void __launch_bounds__(256, 4) gradient_rows_kernel(const T* __restrict__ p,
                                                                const GradArgs a) {

@@ -2592,12 +2592,22 @@ int bfvm_compute_all_gradient_vectors(bfvm_solver* m) {
     auto moderate = [](double d) { return d > 1e-20 && d < 1e20; };
     const bool fast = moderate(m->dx) && moderate(m->dy) && moderate(m->dz);
     const int64_t RS = (int64_t)m->nx * m->S;
+    // Four rows a warp where there are rows enough for it, else a row a block:
+    // time of the rows one by one over time of four at once, 188 meshes: below
+    // 27 blocks of a row an SM 0.54 to 1.02 (50^3 x 4 0.83, 32^3 x 1 0.71), from
+    // there on 0.94 to 1.6 (64^3 x 1 1.09, 80^3 x 4 1.20, 256^3 x 4 1.31); fewer
+    // than four rows a plane 0.5 to 0.9.
+    const bool one = (m->ny < bfvm::kGradRows ||
+                      blocks_for(RS, 256) * m->ny * m->nz < 27 * (int64_t)m->num_sms) &&
+                     m->ny <= 65535 && m->nz <= 65535;
     const dim3 grid((unsigned)blocks_for(RS, 256),
-                    (unsigned)std::min<int64_t>(blocks_for(m->ny, bfvm::kGradRows), 65535),
+                    (unsigned)std::min<int64_t>(blocks_for(m->ny, one ? 1 : bfvm::kGradRows), 65535),
                     std::min(m->nz, 65535));
     with_types(m, [&](auto t, auto) {
       using T = decltype(t);
-      auto k = fast ? bfvm::gradient_rows_kernel<T, true> : bfvm::gradient_rows_kernel<T, false>;
+      auto k = one    ? bfvm::gradient_row_kernel<T>
+               : fast ? bfvm::gradient_rows_kernel<T, true>
+                      : bfvm::gradient_rows_kernel<T, false>;
       const bfvm::GradArgs a{RS, m->ny, m->nz, m->S, dx, dy, dz, m->d_grad.as<double>()};
       k<<<grid, 256, 0, m->stream>>>(m->p.as<T>(), a);
     });

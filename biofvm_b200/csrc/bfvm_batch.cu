@@ -905,13 +905,16 @@ std::string plan_key(const bfvm_batch* b, double dt, int nsteps, int flags) {
     for (const bfvm_solver* m : b->inst) {
       for (int a = 0; a < 3; ++a) {
         // the kernel that sweeps the axis (the closed-form one at its chunk
-        // length, or the axis's own choice) and the chunk length the
-        // Dirichlet segments it reads are laid out for
+        // length, or the axis's own choice), the chunk length the Dirichlet
+        // segments it reads are laid out for, and the setup: a tabulated
+        // kernel's chunk tables follow a new one only when its sweep is
+        // enqueued, which a replay does not do
         const Axis& A = m->axis[a];
-        const int v[9] = {A.ch,     A.tw,    A.minb,
-                          A.kind,   m->chunk_nslots[a],
-                          A.stages, A.build, closed_axis(m, a) ? closed_axis_chunk(m, a) : 0,
-                          a < 2 ? m->dir_ch[a] : 0};
+        const bool closed = closed_axis(m, a);
+        const int64_t v[10] = {A.ch,     A.tw,    A.minb,
+                               A.kind,   m->chunk_nslots[a],
+                               A.stages, A.build, closed ? closed_axis_chunk(m, a) : 0,
+                               a < 2 ? m->dir_ch[a] : 0, closed ? 0 : m->setups};
         k.append(reinterpret_cast<const char*>(v), sizeof v);
       }
       const int64_t v[13] = {m->path, m->fuse_sources, m->precision, m->n_agents,

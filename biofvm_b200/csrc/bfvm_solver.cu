@@ -215,6 +215,7 @@ void thomas_setup(bfvm_solver* m, double dt) {
   closed_setup(m);
   m->grid_tab_ok = false;
   m->setup_done = true;
+  ++m->setups;
 }
 
 // Chunk tables of one axis for its current chunk length (rebuilt when the

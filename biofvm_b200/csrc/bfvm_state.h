@@ -164,6 +164,7 @@ struct bfvm_solver {
   // Thomas coefficients (computed once, BioFVM_solvers.cpp:87,172), with the
   // dt and coefficients they were computed from
   bool setup_done = false;
+  int64_t setups = 0;  // Thomas setups so far
   double setup_dt = 0.0;
   std::vector<double> setup_D, setup_decay;
   bfvm_rt::DevBuf coef[3];  // per axis: inv_den, fwd, bwd [n*S] then c1 [S], in the sweep precision

@@ -2,12 +2,14 @@
 branches: the captured graph must follow the kernel that sweeps each axis and
 the chunk length its Dirichlet segments are laid out for.  Against the oracle
 at the suite's bar for one instance (1e-12 relative max-norm)."""
+import dataclasses
+
 import numpy as np
 import pytest
 
 from biofvm_b200 import Batch, Solver, load_scenario
 from biofvm_b200 import workloads as W
-from biofvm_b200._abi import BATCH_BRANCHES
+from biofvm_b200._abi import BATCH_BRANCHES, PATH_GENERIC, PATH_TMA
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +56,38 @@ def test_a_member_changes_its_sweeps_between_two_steps(shape, S, change):
     for scn, p in zip(scns, got):
         err = O.max_rel_err(p, O.oracle_run(scn, 4, 7))
         assert np.all(err <= 1e-12), (scn.shape, err)
+
+
+@pytest.mark.parametrize("route", ["default", "configured", "tma", "register"])
+def test_new_coefficients_between_two_steps(route):
+    """The diffusion setup is reset and made anew from other coefficients: the
+    graph's kernels must read the new tables, tabulated ones among them."""
+    scns = [W.mixed_small(shape=(24, 40, 20), S=2, n_agents=100, seed=31),
+            W.mixed_small(shape=(20, 30, 10), S=1, n_agents=50, seed=3)]
+    sols = [Solver(0) for _ in scns]
+    try:
+        for sv, scn in zip(sols, scns):
+            load_scenario(sv, scn)
+        if route == "configured":
+            sols[0].set_sweep_config(2, 8, 16)
+        elif route != "default":
+            sols[0].set_kernel_path(PATH_TMA if route == "tma" else PATH_GENERIC)
+        with Batch(0) as bt:
+            for sv in sols:
+                bt.add(sv)
+            bt.set_mode(BATCH_BRANCHES)
+            for _ in range(2):  # the second replays what the first one's tables settled
+                bt.step(scns[0].dt, 2)
+            bt.synchronize()
+            scn = dataclasses.replace(scns[0], D=scns[0].D[::-1] * 3.0, decay=scns[0].decay + 0.5,
+                                      p0=sols[0].get_densities())
+            sols[0].set_coefficients(scn.D, scn.decay)
+            sols[0].reset_diffusion_setup()
+            bt.step(scn.dt, 2)
+            bt.synchronize()
+            err = O.max_rel_err(sols[0].get_densities(), O.oracle_run(scn, 2, 7))
+            other = O.max_rel_err(sols[1].get_densities(), O.oracle_run(scns[1], 6, 7))
+    finally:
+        for sv in sols:
+            sv.close()
+    assert np.all(err <= 1e-12) and np.all(other <= 1e-12), (err, other)

@@ -1332,8 +1332,8 @@ void sweep(bfvm_solver* m, int ax, int fuse, double dt, int64_t z0, int64_t z1) 
     if (path != BFVM_PATH_GENERIC) {
       // build the chunk tables first: the plans size shared memory from them
       chunk_view<CT>(m, ax);
-      // AUTO: the register kernel for x (measured fastest there), TMA tiles
-      // for y and z
+      // AUTO, where a tabulated kernel sweeps: the register kernel for x, TMA
+      // tiles for y and z
       if (path == BFVM_PATH_AUTO && ax == 0) {
         launch_sweep<T, CT>(m, ax, fuse, dt, z0, z1);
         return;

@@ -339,12 +339,15 @@ void tile_kernel(bfvm_solver* m, const CUtensorMap& map, const bfvm::ClosedTileA
   require(per_sm > 0, "sweep kernel does not fit on an SM", BFVM_ERR_STATE);
   // One block per place on the device, except for rows where a place gets many
   // tiles: there several blocks, of a dozen tiles each, follow one another, so
-  // that no SM is left with the slow ones at the end.  Alone on the device, x
-  // 456 -> 430 us at 256^3 x 10 (73 tiles a place) and 1404 -> 1320 at 512^3 x
-  // 8 FP32; 126.7 -> 127.8 at 256^3 x 4 with 27 a place; y and z do not gain.
+  // that no SM is left with the slow ones at the end.  x alone on the device, time
+  // with one block a place over time with several, at 28, 37, 48, 60 and 72 tiles
+  // a place: FP64 256 points x 10 1.03, 1.03, 1.04, 1.05, 1.07, 192 x 4 1.01, 1.02,
+  // 1.04, 1.06, 1.06; FP32 512 x 8 1.00, 0.99, 0.99, 0.98, 1.00, then at 110, 160,
+  // 240 and 400 1.00, 1.00, 1.01, 1.02; FP32 in FP64 arithmetic 256 x 4 0.98 from
+  // 28 to 110, 1.00, 1.00, 1.01 after.  y and z do not gain.
   const uint32_t tiles = a.ntiles - a.tile0, places = (uint32_t)per_sm * m->num_sms;
-  const uint32_t each = tiles / places;
-  const dim3 grid(std::min(tiles, places * (ROWS && each >= 36 ? std::min(8u, each / 12) : 1)));
+  const uint32_t each = tiles / places, many = sizeof(T) == 8 ? 36 : 160;
+  const dim3 grid(std::min(tiles, places * (ROWS && each >= many ? std::min(8u, each / 12) : 1)));
   k<<<grid, block, smem, m->stream>>>(map, a);
   check_launch(m);
 }
